@@ -116,7 +116,7 @@ int vrg_ctx_synchronize(vrg_ctx *ctx);
 int vrg_ctx_set_timing(vrg_ctx *ctx, int enable);
 /* Accumulated device time and launch count of kernel `name` since the last
  * reset; names: "trace_mask", "trace_closest", "trace_lines",
- * "direct_luxels", "direct_points", "transfer_rows", "transfer_rows_sorted",
+ * "sky_map", "direct_luxels", "direct_points", "transfer_rows", "transfer_rows_sorted",
  * "transfer_gather",
  * "bounce_init", "bounce_spmv", "bounce_reduce", "batch_gather",
  * "batch_bounce_init", "batch_spmv", "batch_reduce", "relight_gather",

@@ -31,6 +31,7 @@ constexpr int kGraphBounces = 8;
 // What the batched kernels read of one scene.
 struct BatchDesc {
     DevScene scene;
+    SkyView sky;
     const DevLight *lights;
     const FaceRec *faces;
     const int64_t *luxel_off;
@@ -66,7 +67,7 @@ __device__ __forceinline__ int upper_segment(const int64_t *__restrict__ start, 
 // Work items: segments [0, E) are scene e's luxel supersamples (ss per
 // luxel, in luxel order), segments [E, 2E) scene e's leaf-patch points.
 // OPT: walk options (kOptShRay or none); MINB: resident blocks per SM.
-template <int OPT, int MINB>
+template <bool MAP, int OPT, int MINB>
 __global__ void __launch_bounds__(kThreads, MINB) k_batch_gather(
     const BatchDesc *__restrict__ descs, const int64_t *__restrict__ seg, int nscenes, int ss,
     uint64_t seed, unsigned long long *__restrict__ work, unsigned long long *__restrict__ ray_count) {
@@ -113,7 +114,7 @@ __global__ void __launch_bounds__(kThreads, MINB) k_batch_gather(
                 ny = __ldg(n + 1);
                 nz = __ldg(n + 2);
             }
-            gather_point<kSkyTrace, OPT>(d->scene, d->lights, d->nl, px, py, pz, nx, ny, nz, r, g, b, rays);
+            gather_point<kSkyTrace, OPT, kWallAny, MAP>(d->scene, d->sky, d->lights, d->nl, px, py, pz, nx, ny, nz, r, g, b, rays);
             if (!luxel_item) {
                 float *o = d->pout + 3 * local;
                 o[0] = r;
@@ -275,6 +276,7 @@ BatchDesc make_desc(vrg_env *env) {
     BatchDesc d;
     memset(&d, 0, sizeof d);
     d.scene = scene_view(env);
+    d.sky = sky_view(env);
     d.lights = env->d_lights.as<DevLight>();
     d.faces = env->d_faces.as<FaceRec>();
     d.luxel_off = env->d_luxel_offset.as<int64_t>();
@@ -346,6 +348,18 @@ int vrg_batch_bake(vrg_batch *b, int32_t supersamples, uint64_t seed, int32_t ma
         const int rc = prepare_env(env);
         if (rc != VRG_OK) return rc;
     }
+    // the sky maps serve the launch when every scene has them
+    std::vector<int64_t> points(E);
+    int64_t all_points = 0, repay = 0;
+    for (int e = 0; e < E; e++) {
+        const vrg_env *env = b->envs[e];
+        points[e] = (env->luxel_offset.empty() ? 0 : env->luxel_offset.back()) * supersamples +
+                    (int64_t)env->patches.leaf_patch.size();
+        all_points += points[e];
+        repay += sky_map_points(env);
+    }
+    bool map = true;
+    for (int e = 0; e < E; e++) map = use_sky_map(b->envs[e], points[e], all_points >= repay) && map;
     std::vector<BatchDesc> descs(E);
     std::vector<int64_t> seg(2 * E + 1, 0), rstart(E + 1, 0);
     for (int e = 0; e < E; e++) {
@@ -379,8 +393,9 @@ int vrg_batch_bake(vrg_batch *b, int32_t supersamples, uint64_t seed, int32_t ma
     // the walk constants in shared memory at 9 or 8; the same results)
     using GatherKernel = void (*)(const BatchDesc *, const int64_t *, int, int, uint64_t, unsigned long long *,
                                   unsigned long long *);
-    const GatherKernel gvar[3] = {k_batch_gather<0, 8>, k_batch_gather<kOptShRay, 9>,
-                                  k_batch_gather<kOptShRay, 8>};
+    const GatherKernel gvar[3] = {map ? k_batch_gather<true, 0, 8> : k_batch_gather<false, 0, 8>,
+                                  map ? k_batch_gather<true, kOptShRay, 9> : k_batch_gather<false, kOptShRay, 9>,
+                                  map ? k_batch_gather<true, kOptShRay, 8> : k_batch_gather<false, kOptShRay, 8>};
     const int64_t items = seg[2 * E];
     int64_t tris = 0;
     for (vrg_env *env : b->envs) tris += env->geom.ntris;

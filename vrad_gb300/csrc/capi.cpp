@@ -677,6 +677,13 @@ int vrg_env_set_faces(vrg_env *env, int32_t nfaces, const float *corner, const f
         r.nv = nv[f];
         r.pad0 = r.pad1 = 0;
     }
+    // faces whose corners reach past the scene's largest coordinate have
+    // sample points the sky maps' margins do not cover
+    const float reach = 1.01f * env->geom.scale + 0.5f;
+    env->faces_inside = true;
+    for (int64_t i = 0; i < 3 * (int64_t)nfaces; i++)
+        for (const float c : {corner[i], corner[i] + u[i], corner[i] + v[i], corner[i] + u[i] + v[i]})
+            env->faces_inside = env->faces_inside && std::fabs(c) <= reach && std::fabs(normal[i]) <= 2.0f;
     TRY(upload(ctx, env->d_faces, recs.data(), recs.size() * sizeof(FaceRec)));
     TRY(upload(ctx, env->d_luxel_offset, env->luxel_offset.data(), env->luxel_offset.size() * 8));
     TRY(upload(ctx, env->d_tri_face, env->tri_face.data(), std::max<size_t>(1, env->tri_face.size()) * 4));
@@ -907,7 +914,7 @@ int vrg_env_gather_patch_direct(vrg_env *env, float *out_rgb) {
     const int64_t nl = (int64_t)env->patches.leaf_patch.size();
     VRG_CUDA(ctx, env->d_leaf_direct.reserve(12 * std::max<int64_t>(nl, 1)));
     TRY(launch_gather_points(env, env->d_patch_pts.as<float>(), env->d_patch_nrm.as<float>(), nl,
-                             env->d_leaf_direct.as<float>(), nullptr));
+                             env->d_leaf_direct.as<float>(), nullptr, true));
     if (out_rgb) TRY(download(ctx, out_rgb, env->d_leaf_direct, 12 * nl));
     TRY(sync(ctx));
     env->have_patch_direct = true;

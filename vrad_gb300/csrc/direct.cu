@@ -30,9 +30,9 @@ static_assert(kThreads <= kShRayLanes, "kOptShRay keeps one slot per thread of a
 // TILE walks each face's luxels in 4 x 2 tiles (tile_luxel) instead of row
 // order; the output is the same, each luxel written by the lane holding its
 // first sample.  WM is the scene's wall layout (slots or cells).
-template <int FETCH, int OPT = 0, bool TILE = false, int WM = kWallSlotsOnly, int MINB = 8>
+template <bool MAP, int FETCH, int OPT = 0, bool TILE = false, int WM = kWallSlotsOnly, int MINB = 8>
 __global__ void __launch_bounds__(kThreads, MINB) k_direct_luxels(
-    DevScene s, const DevLight *__restrict__ lights, int nl, const FaceRec *__restrict__ faces,
+    DevScene s, SkyView sv, const DevLight *__restrict__ lights, int nl, const FaceRec *__restrict__ faces,
     const int64_t *__restrict__ off, int nfaces, int64_t nlux, int ss, uint64_t seed,
     float *__restrict__ out, const float *__restrict__ pts, const float *__restrict__ nrm, int64_t npts,
     float *__restrict__ pout, unsigned long long *__restrict__ ray_count,
@@ -85,7 +85,7 @@ __global__ void __launch_bounds__(kThreads, MINB) k_direct_luxels(
             ny = fr.normal.y;
             nz = fr.normal.z;
         }
-        if (gi < total) gather_point<kSkyTrace, OPT, WM>(s, lights, nl, px, py, pz, nx, ny, nz, r, g, b, rays);
+        if (gi < total) gather_point<kSkyTrace, OPT, WM, MAP>(s, sv, lights, nl, px, py, pz, nx, ny, nz, r, g, b, rays);
         if (is_pt) {
             const int64_t i = gi - nsamp;
             pout[3 * i] = r;
@@ -114,8 +114,9 @@ __global__ void __launch_bounds__(kThreads, MINB) k_direct_luxels(
     if ((threadIdx.x & 31) == 0 && ray_count) atomicAdd(ray_count, w);
 }
 
+template <bool MAP>
 __global__ void __launch_bounds__(kThreads, 8) k_direct_points(
-    DevScene s, const DevLight *__restrict__ lights, int nl, const float *__restrict__ pts,
+    DevScene s, SkyView sv, const DevLight *__restrict__ lights, int nl, const float *__restrict__ pts,
     const float *__restrict__ nrm, int64_t n, float *__restrict__ out,
     unsigned long long *__restrict__ ray_count) {
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -124,7 +125,7 @@ __global__ void __launch_bounds__(kThreads, 8) k_direct_points(
         const int64_t i = base + threadIdx.x;
         if (i < n) {
             float r, g, b;
-            gather_point<kSkyTrace>(s, lights, nl, __ldg(pts + 3 * i), __ldg(pts + 3 * i + 1), __ldg(pts + 3 * i + 2),
+            gather_point<kSkyTrace, 0, kWallAny, MAP>(s, sv, lights, nl, __ldg(pts + 3 * i), __ldg(pts + 3 * i + 1), __ldg(pts + 3 * i + 2),
                          __ldg(nrm + 3 * i), __ldg(nrm + 3 * i + 1), __ldg(nrm + 3 * i + 2), r, g, b, rays);
             out[3 * i] = r;
             out[3 * i + 1] = g;
@@ -164,7 +165,7 @@ void pack_lights(const std::vector<vrg_light> &src, std::vector<float4> &dst) {
 // A persistent launch of kernel k: one wave of the blocks k keeps resident
 // per SM, or fewer when the work is small.
 template <class K>
-void launch_direct(K k, int64_t need, int sms, cudaStream_t st, const DevScene &s, const DevLight *lights, int nl,
+void launch_direct(K k, int64_t need, int sms, cudaStream_t st, const DevScene &s, const SkyView &sv, const DevLight *lights, int nl,
                    const vrg_env *env, int64_t nlux, int ss, uint64_t seed, float *out_rgb, const float *pts,
                    const float *nrm, int64_t npts, float *pts_out, unsigned long long *d_rays,
                    unsigned long long *work) {
@@ -172,7 +173,7 @@ void launch_direct(K k, int64_t need, int sms, cudaStream_t st, const DevScene &
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kThreads, 0) != cudaSuccess || per_sm < 1)
         per_sm = 4;
     const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(need, (int64_t)sms * per_sm));
-    k<<<grid, kThreads, 0, st>>>(s, lights, nl, env->d_faces.as<FaceRec>(), env->d_luxel_offset.as<int64_t>(),
+    k<<<grid, kThreads, 0, st>>>(s, sv, lights, nl, env->d_faces.as<FaceRec>(), env->d_luxel_offset.as<int64_t>(),
                                  env->nfaces, nlux, ss, seed, out_rgb, pts, nrm, npts, pts_out, d_rays, work);
 }
 
@@ -183,13 +184,13 @@ void launch_direct(K k, int64_t need, int sms, cudaStream_t st, const DevScene &
 // walk constants in shared memory at 8, 9 or 10 resident blocks per SM (64,
 // 56 or 48 registers), in plain tiles at 9 blocks, and in tiles with the
 // walk constants and the top of the tree in shared memory at 9 blocks.
-template <int WM>
-void launch_direct_variant(int v, int64_t need, int sms, cudaStream_t st, const DevScene &s,
+template <int WM, bool MAP>
+void launch_direct_variant(int v, int64_t need, int sms, cudaStream_t st, const DevScene &s, const SkyView &sv,
                            const DevLight *lights, int nl, const vrg_env *env, int64_t nlux, int ss,
                            uint64_t seed, float *out_rgb, const float *pts, const float *nrm, int64_t npts,
                            float *pts_out, unsigned long long *d_rays, unsigned long long *work) {
 #define VRG_DIRECT(...) \
-    launch_direct(k_direct_luxels<__VA_ARGS__>, need, sms, st, s, lights, nl, env, nlux, ss, seed, out_rgb, pts, \
+    launch_direct(k_direct_luxels<MAP, __VA_ARGS__>, need, sms, st, s, sv, lights, nl, env, nlux, ss, seed, out_rgb, pts, \
                   nrm, npts, pts_out, d_rays, work)
     switch (v) {
     case 0: VRG_DIRECT(32, 0, false, WM); break;
@@ -217,7 +218,9 @@ int launch_gather_luxels(vrg_env *env, int ss, uint64_t seed, float *out_rgb,
     VRG_CUDA(ctx, env->d_work.reserve(256));
     unsigned long long *work = env->d_work.as<unsigned long long>() + 1;
     const int64_t need = (nlux * ss + npts + kThreads - 1) / kThreads;
+    const bool map = use_sky_map(env, nlux * ss + npts);
     const DevScene s = scene_view(env);
+    const SkyView sv = sky_view(env);
     const DevLight *lights = env->d_lights.as<DevLight>();
     const int nl = (int)env->lights.size();
     // the variants of launch_direct_variant, picked per bucket, built for the
@@ -228,12 +231,14 @@ int launch_gather_luxels(vrg_env *env, int ss, uint64_t seed, float *out_rgb,
         if (e != cudaSuccess) return e;
         cudaEvent_t ev = nullptr;
         timing_begin(ctx, "direct_luxels", &ev);
+        auto go = [&](auto variant) {
+            variant(v, need, ctx->num_sms, ctx->stream, s, sv, lights, nl, env, nlux, ss, seed, out_rgb, pts, nrm,
+                    npts, pts_out, d_rays, work);
+        };
         if (env->wall_layout == 0)
-            launch_direct_variant<kWallSlotsOnly>(v, need, ctx->num_sms, ctx->stream, s, lights, nl, env, nlux, ss,
-                                                  seed, out_rgb, pts, nrm, npts, pts_out, d_rays, work);
+            go(map ? launch_direct_variant<kWallSlotsOnly, true> : launch_direct_variant<kWallSlotsOnly, false>);
         else
-            launch_direct_variant<kWallCellsOnly>(v, need, ctx->num_sms, ctx->stream, s, lights, nl, env, nlux, ss,
-                                                  seed, out_rgb, pts, nrm, npts, pts_out, d_rays, work);
+            go(map ? launch_direct_variant<kWallCellsOnly, true> : launch_direct_variant<kWallCellsOnly, false>);
         e = cudaGetLastError();
         timing_end(ctx, "direct_luxels", ev);
         return e;
@@ -242,13 +247,14 @@ int launch_gather_luxels(vrg_env *env, int ss, uint64_t seed, float *out_rgb,
 }
 
 int launch_gather_points(vrg_env *env, const float *pts, const float *nrm, int64_t n,
-                         float *out_rgb, unsigned long long *d_rays) {
+                         float *out_rgb, unsigned long long *d_rays, bool on_faces) {
     vrg_ctx *ctx = env->ctx;
     if (n <= 0) return VRG_OK;
+    const bool map = on_faces && use_sky_map(env, n);
     cudaEvent_t ev = nullptr;
     timing_begin(ctx, "direct_points", &ev);
-    k_direct_points<<<grid_for(ctx, n), kThreads, 0, ctx->stream>>>(
-        scene_view(env), env->d_lights.as<DevLight>(), (int)env->lights.size(), pts, nrm, n,
+    (map ? k_direct_points<true> : k_direct_points<false>)<<<grid_for(ctx, n), kThreads, 0, ctx->stream>>>(
+        scene_view(env), sky_view(env), env->d_lights.as<DevLight>(), (int)env->lights.size(), pts, nrm, n,
         out_rgb, d_rays);
     VRG_CUDA(ctx, cudaGetLastError());
     timing_end(ctx, "direct_points", ev);

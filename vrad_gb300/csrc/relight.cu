@@ -71,9 +71,9 @@ __device__ __forceinline__ int seg_of(const int64_t *__restrict__ off, int n, in
 // sky multipliers and the point/spot visibility bits (vis_words words per
 // sample or point), kSkyRead reuses them and traces only the lights flagged
 // in `edited`.
-template <int SKY>
+template <int SKY, bool MAP = false>
 __global__ void __launch_bounds__(kThreads, 8) k_relight_gather(
-    DevScene s, const DevLight *__restrict__ lights, int nl, const FaceRec *__restrict__ faces,
+    DevScene s, SkyView sv, const DevLight *__restrict__ lights, int nl, const FaceRec *__restrict__ faces,
     const int64_t *__restrict__ luxel_off, int nfaces, RelightList list, int ss, uint64_t seed,
     float *__restrict__ lux_out, const float *__restrict__ ppts, const float *__restrict__ pnrm,
     float *__restrict__ pout, float *__restrict__ sky_lux, float *__restrict__ sky_pts, int sky_slots,
@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(kThreads, 8) k_relight_gather(
             const int64_t gsamp = lux * ss + kk;
             float px, py, pz;
             luxel_sample(fr, lux, iu, iv, kk, ss, seed, px, py, pz);
-            gather_point<SKY>(s, lights, nl, px, py, pz, fr.normal.x, fr.normal.y, fr.normal.z, r, g,
+            gather_point<SKY, 0, kWallAny, MAP>(s, sv, lights, nl, px, py, pz, fr.normal.x, fr.normal.y, fr.normal.z, r, g,
                               b, rays, sky_lux + gsamp * sky_slots, vis_lux + gsamp * vis_words, edited);
         } else if (gi < total) {
             const int64_t li = gi - nsamp;
@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(kThreads, 8) k_relight_gather(
                 leaf = __ldg(list.leaf_beg + k) + (li - __ldg(list.leaf_off + k));
             }
             const float *p = ppts + 3 * leaf, *n = pnrm + 3 * leaf;
-            gather_point<SKY>(s, lights, nl, __ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(n), __ldg(n + 1),
+            gather_point<SKY, 0, kWallAny, MAP>(s, sv, lights, nl, __ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(n), __ldg(n + 1),
                               __ldg(n + 2), r, g, b, rays, sky_pts + leaf * sky_slots,
                               vis_pts + leaf * vis_words, edited);
             pout[3 * leaf] = r;
@@ -505,8 +505,9 @@ int relight_prepare(vrg_env *env, int32_t ss, uint64_t seed, int32_t max_bounces
     const int64_t items = nlux * ss + nl;
     cudaEvent_t ev = nullptr;
     timing_begin(ctx, "relight_gather", &ev);
-    k_relight_gather<kSkyWrite><<<persistent_blocks(ctx, (const void *)k_relight_gather<kSkyWrite>, items), kThreads, 0, st>>>(
-        scene_view(env), env->d_lights.as<DevLight>(), (int)env->lights.size(), env->d_faces.as<FaceRec>(),
+    const auto gather = use_sky_map(env, items) ? k_relight_gather<kSkyWrite, true> : k_relight_gather<kSkyWrite>;
+    gather<<<persistent_blocks(ctx, (const void *)gather, items), kThreads, 0, st>>>(
+        scene_view(env), sky_view(env), env->d_lights.as<DevLight>(), (int)env->lights.size(), env->d_faces.as<FaceRec>(),
         env->d_luxel_offset.as<int64_t>(), env->nfaces, all, ss, seed, env->d_bake_rgb.as<float>(),
         env->d_patch_pts.as<float>(), env->d_patch_nrm.as<float>(), env->d_leaf_direct.as<float>(),
         env->d_sky_lux.as<float>(), env->d_sky_pts.as<float>(), sky, env->d_vis_lux.as<uint32_t>(),
@@ -720,7 +721,7 @@ int issue_relight(vrg_env *env, const RelightPlan &p, int32_t max_iters, float t
     const int64_t items = hs[nf] + hl[nf];
     if (items > 0) {
         k_relight_gather<kSkyRead><<<persistent_blocks(ctx, (const void *)k_relight_gather<kSkyRead>, items), kThreads, 0, st>>>(
-            scene_view(env), env->d_lights.as<DevLight>(), (int)p.table.size(), env->d_faces.as<FaceRec>(),
+            scene_view(env), SkyView{}, env->d_lights.as<DevLight>(), (int)p.table.size(), env->d_faces.as<FaceRec>(),
             env->d_luxel_offset.as<int64_t>(), F, list, ss, env->relight_seed, env->d_bake_rgb.as<float>(),
             env->d_patch_pts.as<float>(), env->d_patch_nrm.as<float>(), env->d_leaf_direct.as<float>(),
             env->d_sky_lux.as<float>(), env->d_sky_pts.as<float>(), env->sky_slots,

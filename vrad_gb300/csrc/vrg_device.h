@@ -80,6 +80,34 @@ __host__ __device__ inline const uint32_t *wall_table(const DevScene &s) {
     return reinterpret_cast<const uint32_t *>(s.leaf_edges + 2 * (s.leaf_edges - s.leaf_planes));
 }
 
+// Sky maps.  The sky-ambient light sends lines in 162 fixed directions, so
+// per direction the scene is a picture seen along parallel lines: points are
+// sheared along the direction onto the plane of the other two axes (cell
+// coordinates cu, cv) and keep their depth along the direction's largest
+// axis, 65,000 levels over the scene.  A cell stores two conservative
+// depths.  A plain cell: below the first (low half; 0: none) an opaque
+// triangle covering the whole cell, with no sky triangle before it, stops
+// every line; above the second (high half, in steps of two) no opaque
+// triangle is left.  A cell whose sky lies before its covering triangle
+// (kSkyPast: a line going down, away from the sky it would come from): the
+// covering triangle stops every line that starts between the second depth,
+// past all sky, and the first.  Any other line tests the cell's list: the
+// triangles over the cell that reach above the first depth or, in a
+// kSkyPast cell, start before the second (sky triangles only where an opaque
+// one reaches past them: kSkyCellFlag).
+// All bounds are widened by a margin far beyond the rounding of the exact
+// ray/triangle test, so that a line's answer is the walk's.
+struct SkyView {
+    const uint32_t *bound;  // per direction and cell: first depth | second / 2 << 16 | kSkyPast
+    const uint2 *info;      // first pool entry, entries | kSkyCellFlag
+    const uint2 *pool;      // leaf-record index, depth above which the triangle is clear; per cell
+                            // in descending order of that depth
+    const float4 *dirs;     // per direction: cu, cv and depth as dot products (xyz . p + w)
+    int32_t n;              // cells per axis
+};
+constexpr uint32_t kSkyPast = 1u << 31;      // in `bound`
+constexpr uint32_t kSkyCellFlag = 1u << 31;  // the cell's list holds sky triangles
+
 // The top table holds the first kTopNodes nodes of a breadth-first walk from
 // the root, children pairs kept adjacent.  A child word there whose index
 // has kTopRef set points into the table instead of the node array, so a

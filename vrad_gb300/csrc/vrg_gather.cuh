@@ -5,17 +5,11 @@
 #include <cstdint>
 
 #include "../../include/vradgpu.h"
-#include "anorms_table.h"
 #include "vrg_device.h"
+#include "vrg_sky.cuh"
 #include "vrg_trace.cuh"
 
 namespace vrg {
-
-// The 162 sky directions (one copy per translation unit).
-static __constant__ float c_anorms[kNumAnorms * 3] = VRG_ANORMS_INIT;
-
-
-
 
 // Device copy of a light: five 16-byte words.
 struct alignas(16) DevLight {
@@ -51,10 +45,12 @@ __device__ __forceinline__ uint64_t splitmix(uint64_t seed, uint64_t i) {
 // The accumulation order and arithmetic are the same in all modes, so a
 // relight that re-traces only edited lights is bit-identical to a full
 // gather with the edited table.
+// MAP answers the sky ambient's lines from the scene's sky maps (sv) instead
+// of walking them; the results are the same.
 enum SkyMode { kSkyTrace = 0, kSkyWrite = 1, kSkyRead = 2 };
 
-template <int SKY, int OPT = 0, int WM = kWallAny>
-static __device__ void gather_point(const DevScene &s, const DevLight *__restrict__ lights, int nl,
+template <int SKY, int OPT = 0, int WM = kWallAny, bool MAP = false>
+static __device__ void gather_point(const DevScene &s, const SkyView &sv, const DevLight *__restrict__ lights, int nl,
                                     float px, float py, float pz, float nx, float ny, float nz,
                                     float &r, float &g, float &b, uint32_t &rays,
                                     float *__restrict__ sky = nullptr, uint32_t *__restrict__ vis = nullptr,
@@ -131,8 +127,10 @@ static __device__ void gather_point(const DevScene &s, const DevLight *__restric
                                              radd(pz, rmul(dz, kMaxTraceLength)));
                     if (!line_occluded<OPT, WM>(s, L, -1)) m = cosr;
                 }
+            } else if (MAP) {
+                m = sky_fraction(s, sv, px, py, pz, nx, ny, nz, rays);
             } else {
-                float sw = 0.0f, sv = 0.0f;
+                float sw = 0.0f, sum = 0.0f;
                 for (int j = 0; j < kNumAnorms; j++) {
                     const float ax = c_anorms[3 * j], ay = c_anorms[3 * j + 1], az = c_anorms[3 * j + 2];
                     const float w = dot3r(nx, ny, nz, ax, ay, az);
@@ -142,9 +140,9 @@ static __device__ void gather_point(const DevScene &s, const DevLight *__restric
                     const Line L = make_line(px, py, pz, radd(px, rmul(ax, kMaxTraceLength)),
                                              radd(py, rmul(ay, kMaxTraceLength)),
                                              radd(pz, rmul(az, kMaxTraceLength)));
-                    if (!line_occluded<OPT, WM>(s, L, -1)) sv = radd(sv, w);
+                    if (!line_occluded<OPT, WM>(s, L, -1)) sum = radd(sum, w);
                 }
-                if (sw > 0.0f) m = rdiv(sv, sw);
+                if (sw > 0.0f) m = rdiv(sum, sw);
             }
             if (SKY == kSkyWrite) *sky++ = m;
             if (m >= 0.0f) {

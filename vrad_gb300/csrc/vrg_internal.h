@@ -86,6 +86,8 @@ struct vrg_ctx {
     bool autotune = true;
     uint64_t hbm_reserve = (uint64_t)1 << 30;  // kept free when admitting a relight scene
     int32_t xfer_table_limit = 7168;            // distinct targets per transfer row held in shared memory
+    std::mutex sky_mu;           // held through a sky-map build
+    vrg::DevBuf sky_scratch;     // its scratch, at most 64 MiB between builds
     std::map<std::string, int> tuned;                   // bucket key -> variant
     std::map<std::string, std::vector<double>> tune_ms;  // bucket key -> variant times
 };
@@ -157,6 +159,11 @@ struct vrg_env {
     bool cover_ready = false;
     int32_t n_transparent = 0;
 
+    // sky maps (skymap.cu): cells per axis (0: not built, -1: cannot be)
+    int32_t sky_n = 0;
+    int64_t sky_demand = 0;  // sample points gathered without the maps
+    vrg::DevBuf d_sky_cells, d_sky_pool;
+
     // lights
     std::vector<vrg_light> lights;
     vrg::DevBuf d_lights;
@@ -166,6 +173,7 @@ struct vrg_env {
     std::vector<float> f_corner, f_u, f_v, f_normal, f_luxscale, f_refl, f_base;
     std::vector<int32_t> f_nu, f_nv, tri_face;
     std::vector<int64_t> luxel_offset;
+    bool faces_inside = false;  // every face lies within the scene's coordinates
     vrg::DevBuf d_faces, d_luxel_offset, d_tri_face;
 
     // patches / transfers / bounce
@@ -257,13 +265,19 @@ int launch_trace_closest(vrg_env *env, const float *orig, const float *dir, cons
                          const float *tmax, int64_t n, int32_t skip_id, int32_t *hit, float *t);
 int launch_test_lines(vrg_env *env, const float *start, const float *stop, int64_t n,
                       int32_t skip_id, float *frac);
+// Sky maps: whether the sky-ambient lines of `points` sample points on the
+// scene's faces go through the maps (built here when the points repay it), and
+// the maps as the kernels read them.
+bool use_sky_map(vrg_env *env, int64_t points, bool repaid = false);
+int64_t sky_map_points(const vrg_env *env);  // sample points that repay building the maps
+SkyView sky_view(const vrg_env *env);
 // Luxel samples of every face, then (optionally) npts extra sample points
 // in the same persistent launch.
 int launch_gather_luxels(vrg_env *env, int ss, uint64_t seed, float *out_rgb,
                          unsigned long long *d_rays, const float *pts = nullptr,
                          const float *nrm = nullptr, int64_t npts = 0, float *pts_out = nullptr);
 int launch_gather_points(vrg_env *env, const float *pts, const float *nrm, int64_t n,
-                         float *out_rgb, unsigned long long *d_rays);
+                         float *out_rgb, unsigned long long *d_rays, bool on_faces = false);
 void pack_lights(const std::vector<vrg_light> &src, std::vector<float4> &dst);
 int run_make_transfers(vrg_env *env, const float *dirs_local, int32_t k);
 int run_bounce(vrg_env *env, int32_t max_bounces, float rel_tol, int32_t *bounces,

@@ -47,6 +47,9 @@ constexpr int kShRayLanes = 128;
 // and a warp-wide mask of the lanes out of work, one ballot per round
 // instead of two.
 constexpr int kOptOneVote = 64;
+// kOptSign: a triangle test gives up before its division when the plane lies
+// behind the origin (the quotient's sign is known).
+constexpr int kOptSign = 128;
 
 // Shared-memory copy of the scene's top table, for kernels walking with
 // kOptTop (allocated only in kernels that use it).
@@ -254,7 +257,12 @@ __device__ __forceinline__ bool tri_test(const DevScene &s, const Ray &ray, floa
                                          int32_t &best, float &best_t) {
     const float den = dot3r(w0.x, w0.y, w0.z, ray.dx, ray.dy, ray.dz);
     const float on = dot3r(w0.x, w0.y, w0.z, ray.ox, ray.oy, ray.oz);
-    const float t = rdiv(rsub(w0.w, on), den);
+    const float num = rsub(w0.w, on);
+    if (OPT & kOptSign) {
+        // signs differ: t < 0 (above 1e-30 the quotient does not round to -0)
+        if (((__float_as_uint(num) ^ __float_as_uint(den)) >> 31) && fabsf(num) > 1e-30f) return false;
+    }
+    const float t = rdiv(num, den);
     if (!(t >= tmin && t < tmax)) return false;
     if (MODE != kAny && !(t <= best_t)) return false;
     const float4 *ed = s.leaf_edges + 2 * k;
