@@ -15,7 +15,6 @@ namespace {
 
 constexpr int kThreads = 128;
 constexpr int kWarps = kThreads / 32;
-constexpr size_t kScratchKept = (size_t)64 << 20;  // scratch a context keeps between builds
 constexpr float kDepthLevels = 65000.0f;  // depths lie in [1, 65001]
 
 // What the kernels read of one triangle: its vertices and the leaf record
@@ -416,7 +415,7 @@ void make_dirs(const vrg_env *env, int n, std::vector<SkyDir> &out) {
 // holds until its kernels are done.
 int build(vrg_env *env, int n) {
     vrg_ctx *ctx = env->ctx;
-    std::lock_guard<std::mutex> scratch(ctx->sky_mu);
+    std::lock_guard<std::mutex> scratch(ctx->scratch_mu);
     cudaStream_t st = ctx->stream;
     const int64_t nt = env->geom.ntris;
     const size_t cells = (size_t)kNumAnorms * n * n;
@@ -456,7 +455,7 @@ int build(vrg_env *env, int n) {
     // scratch [counters | grids | large pairs | triangles | directions]
     const size_t tri_at = (256 + 4 * cells * (has_sky ? 4 : 1) + 4 * (size_t)pairs + 15) & ~(size_t)15;
     const size_t dir_at = tri_at + sizeof(SkyTri) * (size_t)nt;
-    DevBuf &tmp = ctx->sky_scratch;
+    DevBuf &tmp = ctx->scratch;
     VRG_CUDA(ctx, tmp.reserve(dir_at + sizeof(SkyDir) * kNumAnorms));
     SkyTri *d_tris = reinterpret_cast<SkyTri *>(tmp.as<char>() + tri_at);
     SkyDir *d_dirs = reinterpret_cast<SkyDir *>(tmp.as<char>() + dir_at);

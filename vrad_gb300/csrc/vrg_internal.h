@@ -58,6 +58,8 @@ struct DevBuf {
 struct RelightState;  // relight.cu: serial scratch and loop graphs of a scene
 struct BounceGraph;   // bounce.cu: the scene's bounce loop as a graph
 
+constexpr size_t kScratchKept = (size_t)256 << 20;
+
 struct KernelStat {
     double ms = 0.0;
     int64_t launches = 0;
@@ -86,8 +88,10 @@ struct vrg_ctx {
     bool autotune = true;
     uint64_t hbm_reserve = (uint64_t)1 << 30;  // kept free when admitting a relight scene
     int32_t xfer_table_limit = 7168;            // distinct targets per transfer row held in shared memory
-    std::mutex sky_mu;           // held through a sky-map build
-    vrg::DevBuf sky_scratch;     // its scratch, at most 64 MiB between builds
+    // scratch of the sky-map and transfer builds, which hold scratch_mu until
+    // their kernels are done; at most kScratchKept of it is kept between them
+    std::mutex scratch_mu;
+    vrg::DevBuf scratch;
     std::map<std::string, int> tuned;                   // bucket key -> variant
     std::map<std::string, std::vector<double>> tune_ms;  // bucket key -> variant times
 };
@@ -182,6 +186,9 @@ struct vrg_env {
     vrg::DevBuf d_patch_nodes, d_leaf_info, d_face_root;
     vrg::DevBuf d_face_tree;  // int4 per face: see face_tree_ranges (capi.cpp)
     bool have_transfers = false;
+    int32_t tile_tris = -1;       // triangles in d_tile_scene (-1: not made), and to a cluster
+    int32_t tile_per = 0;
+    vrg::DevBuf d_tile_scene;     // the triangles as the tiled transfer rows read them (transfer.cu)
     int64_t nnz = 0;
     int32_t transfer_k = 0;
     int64_t transfer_overflow_rows = 0;  // rows of the last build past the shared-memory row table
