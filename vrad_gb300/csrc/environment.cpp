@@ -3,6 +3,7 @@
 // upload to the device.
 #include <algorithm>
 #include <limits>
+#include <memory>
 #include <cmath>
 #include <cstring>
 #include <thread>
@@ -142,6 +143,12 @@ int vrg_env_setup_acceleration_structure(vrg_env *env) {
         }
         g.scale = scale;
     });
+    // so is the hierarchy of the line queries (device contexts only)
+    std::vector<BvhNode> bvh;
+    std::thread hierarchy([env, n, ctx, &bvh]() {
+        if (ctx->host_only || n >= (int64_t)1 << 27) return;
+        build_bvh(env->xyz, env->bvh_order, bvh);
+    });
     int rc = VRG_OK;
     if (on_device) {
         const cudaError_t e = cudaSetDevice(ctx->device);
@@ -150,6 +157,13 @@ int vrg_env_setup_acceleration_structure(vrg_env *env) {
         build_walk_tree(env->xyz, env->min_bound, env->max_bound, env->walk_costs, env->walk_tree);
     }
     records.join();
+    // joined where its order is needed, or on the way out
+    struct Join {
+        std::thread &t;
+        ~Join() {
+            if (t.joinable()) t.join();
+        }
+    } join_hierarchy{hierarchy};
     if (rc != VRG_OK) return rc;
     // A walk pushes at most one subtree per inner node on its path, so a tree
     // whose paths hold fewer inner nodes than the device's stack has entries
@@ -259,8 +273,15 @@ int vrg_env_setup_acceleration_structure(vrg_env *env) {
     size_t nw = 6 * (size_t)kWallSlots;
     for (int f = 0; f < 6; f++)
         if (use_cells) nw += wall[f].size();
-    const size_t ne = nr + nw;  // leaf entries + wall slots + wall-cell records
-    std::vector<float4> leaf(3 * ne, make_float4(0, 0, 0, 0));
+    // then the triangles in the order of the hierarchy's leaves
+    hierarchy.join();
+    const size_t nb = env->bvh_order.size(), tri_base = nr + nw;
+    const size_t ne = tri_base + nb;
+    // (the records of unused wall slots are zero, all others written below;
+    // the cell table, counted once it is made, goes after them)
+    std::unique_ptr<float4[]> leaf(new float4[3 * ne]);
+    for (size_t r = nr; r < tri_base; r++)
+        leaf[r] = leaf[ne + 2 * r] = leaf[ne + 2 * r + 1] = make_float4(0, 0, 0, 0);
     auto put = [&](size_t r, int32_t tri) {
         const TriRecord &t = env->tri_records[tri];
         float id_bits, idx_bits;
@@ -274,7 +295,8 @@ int vrg_env_setup_acceleration_structure(vrg_env *env) {
     g.wall_base = (uint32_t)nr;
     g.wall_count = 0;
     g.wall_cell_mask = 0;
-    env->n_wall_records = nw;
+    env->tri_base = (int64_t)tri_base;
+    env->n_extra_records = nw + nb;
     // the cell table: 6 face descriptors of kWallFaceWords words (cell origin
     // and inverse size in the face's two in-plane axes as float bits, cells
     // per axis, offset of the face's cell starts), then per face with walls
@@ -342,27 +364,32 @@ int vrg_env_setup_acceleration_structure(vrg_env *env) {
     }
     {  // the cell table after the edge part (wall_table), padded to whole float4s
         cells.resize((cells.size() + 3) & ~(size_t)3, 0u);
-        const size_t at = leaf.size();
-        leaf.resize(at + cells.size() / 4);
-        memcpy(&leaf[at], cells.data(), cells.size() * sizeof(uint32_t));
     }
     {  // the leaf entries, in parallel chunks
         const unsigned hw = std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
-        const size_t nt = nr < 65536 ? 1 : hw, chunk = (nr + nt - 1) / nt;
+        const size_t nt = nr < 65536 ? 1 : hw, chunk = (nr + nt - 1) / nt, bchunk = (nb + nt - 1) / nt;
         std::vector<std::thread> pool;
         for (size_t w = 1; w < nt; w++)
             pool.emplace_back([&, w]() {
                 for (size_t r = w * chunk; r < std::min(nr, (w + 1) * chunk); r++) put(r, wt.refs[r]);
+                for (size_t i = w * bchunk; i < std::min(nb, (w + 1) * bchunk); i++) put(tri_base + i, env->bvh_order[i]);
             });
         for (size_t r = 0; r < std::min(nr, chunk); r++) put(r, wt.refs[r]);
+        for (size_t i = 0; i < std::min(nb, bchunk); i++) put(tri_base + i, env->bvh_order[i]);
         for (std::thread &t : pool) t.join();
     }
     env->built = true;
     env->cover_ready = false;
     if (ctx->host_only) return VRG_OK;
     VRG_CUDA(ctx, cudaSetDevice(ctx->device));
+    if (!bvh.empty()) {
+        VRG_CUDA(ctx, env->d_bvh.reserve(bvh.size() * sizeof(BvhNode)));
+        VRG_CUDA(ctx, cudaMemcpyAsync(env->d_bvh.ptr, bvh.data(), bvh.size() * sizeof(BvhNode), cudaMemcpyHostToDevice,
+                                      ctx->stream));
+        env->bvh_nodes = (int64_t)bvh.size();
+    }
     VRG_CUDA(ctx, env->d_nodes.reserve(nn * sizeof(uint2)));
-    VRG_CUDA(ctx, env->d_leaf_tris.reserve(leaf.size() * sizeof(float4)));
+    VRG_CUDA(ctx, env->d_leaf_tris.reserve(3 * ne * sizeof(float4) + cells.size() * sizeof(uint32_t)));
     VRG_CUDA(ctx, env->d_tri_ids.reserve((n ? n : 1) * sizeof(int32_t)));
     VRG_CUDA(ctx, env->d_top.reserve(std::max<size_t>(top.size(), 1) * sizeof(uint2)));
     if (!top.empty())
@@ -370,8 +397,10 @@ int vrg_env_setup_acceleration_structure(vrg_env *env) {
                                       cudaMemcpyHostToDevice, ctx->stream));
     VRG_CUDA(ctx, cudaMemcpyAsync(env->d_nodes.ptr, nodes.data(), nn * sizeof(uint2),
                                   cudaMemcpyHostToDevice, ctx->stream));
-    VRG_CUDA(ctx, cudaMemcpyAsync(env->d_leaf_tris.ptr, leaf.data(), leaf.size() * sizeof(float4),
+    VRG_CUDA(ctx, cudaMemcpyAsync(env->d_leaf_tris.ptr, leaf.get(), 3 * ne * sizeof(float4),
                                   cudaMemcpyHostToDevice, ctx->stream));
+    VRG_CUDA(ctx, cudaMemcpyAsync(env->d_leaf_tris.as<float4>() + 3 * ne, cells.data(),
+                                  cells.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, ctx->stream));
     if (n)
         VRG_CUDA(ctx, cudaMemcpyAsync(env->d_tri_ids.ptr, env->ids.data(), n * sizeof(int32_t),
                                       cudaMemcpyHostToDevice, ctx->stream));

@@ -12,6 +12,7 @@
 #include <cmath>
 
 #include "vrg_internal.h"
+#include "vrg_bvh.cuh"
 #include "vrg_trace.cuh"
 
 namespace vrg {
@@ -70,17 +71,20 @@ __device__ __forceinline__ int32_t hit_leaf(const RowFrame &fr, const PatchNode 
     return pn.leaf;
 }
 
-// Target leaf of ray r of a row (-1: no lit face hit).
-template <int OPT>
-__device__ __forceinline__ int32_t row_ray_target(const DevScene &s, const RowFrame &fr,
+// Target leaf of ray r of a row (-1: no lit face hit), walked in the kd tree or
+// the line queries' hierarchy.
+template <bool BVH>
+__device__ __forceinline__ int32_t row_ray_target(const DevScene &s, const BvhView &bv, const RowFrame &fr,
                                                   const PatchNode *__restrict__ pnodes,
                                                   const int32_t *__restrict__ face_root,
                                                   const int32_t *__restrict__ tri_face,
                                                   const float *__restrict__ dirs, int r) {
     float dx, dy, dz, t;
     row_ray(fr, dirs, r, dx, dy, dz);
-    const int32_t h = trace_ray<kClosest, OPT>(s, Ray{fr.qx, fr.qy, fr.qz, dx, dy, dz}, 0.0f, kMaxTraceLength,
-                                               -1, &t);
+    const Ray ray{fr.qx, fr.qy, fr.qz, dx, dy, dz};
+    const int32_t h = BVH ? bvh_trace<kClosest, kOptSign>(s, bv, ray, ray_slack(s.g, fr.qx, fr.qy, fr.qz), 0.0f,
+                                                          kMaxTraceLength, -1, 0.0f, &t)
+                          : trace_ray<kClosest, kOptSkip>(s, ray, 0.0f, kMaxTraceLength, -1, &t);
     return hit_leaf(fr, pnodes, face_root, tri_face, h, t, dx, dy, dz);
 }
 
@@ -168,9 +172,9 @@ __device__ __forceinline__ int write_row(const RowCounts &rc, int limit, int *su
 // writes nnz = -1 and is rebuilt by k_transfer_rows_sorted.  NT threads per
 // block at most; k is a multiple of the block size, so every lane of a warp
 // runs the same rays.
-template <int NT>
+template <int NT, bool BVH>
 __global__ void __launch_bounds__(NT) k_transfer_rows(
-    DevScene s, const LeafInfo *__restrict__ leaves, const FaceRec *__restrict__ faces,
+    DevScene s, BvhView bv, const LeafInfo *__restrict__ leaves, const FaceRec *__restrict__ faces,
     const PatchNode *__restrict__ pnodes, const int32_t *__restrict__ face_root,
     const int32_t *__restrict__ tri_face, const float *__restrict__ dirs, int k, int64_t row0,
     int64_t rows, int nleaves, int stride, int limit, uint32_t *__restrict__ scratch, int64_t scratch_stride,
@@ -184,7 +188,7 @@ __global__ void __launch_bounds__(NT) k_transfer_rows(
         const LeafInfo li = leaves[row];
         const RowFrame fr = row_frame(li, faces[__float_as_int(li.refl.w)]);
         for (int r = tid; r < k; r += nt) {
-            const int32_t target = row_ray_target<kOptSkip>(s, fr, pnodes, face_root, tri_face, dirs, r);
+            const int32_t target = row_ray_target<BVH>(s, bv, fr, pnodes, face_root, tri_face, dirs, r);
             const unsigned peers = __match_any_sync(0xffffffffu, target);
             if (target >= 0 && lane == __ffs(peers) - 1) row_add(rc, target, (uint32_t)__popc(peers));
         }
@@ -663,7 +667,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_transfer_tiles(
 // multiple of the block size.
 template <int NT>
 __global__ void __launch_bounds__(NT) k_transfer_rows_sorted(
-    DevScene s, const LeafInfo *__restrict__ leaves, const FaceRec *__restrict__ faces,
+    DevScene s, BvhView bv, const LeafInfo *__restrict__ leaves, const FaceRec *__restrict__ faces,
     const PatchNode *__restrict__ pnodes, const int32_t *__restrict__ face_root,
     const int32_t *__restrict__ tri_face, const float *__restrict__ dirs, int k,
     const int64_t *__restrict__ row_list, int64_t nlist, int32_t *__restrict__ scratch,
@@ -678,7 +682,7 @@ __global__ void __launch_bounds__(NT) k_transfer_rows_sorted(
         const int64_t row = row_list[j];
         const LeafInfo li = leaves[row];
         const RowFrame fr = row_frame(li, faces[__float_as_int(li.refl.w)]);
-        for (int r = tid; r < k; r += nt) tg[r] = row_ray_target<0>(s, fr, pnodes, face_root, tri_face, dirs, r);
+        for (int r = tid; r < k; r += nt) tg[r] = row_ray_target<true>(s, bv, fr, pnodes, face_root, tri_face, dirs, r);
         __syncthreads();
         for (int size = 2; size <= k; size <<= 1) {
             for (int stride = size >> 1; stride > 0; stride >>= 1) {
@@ -1007,23 +1011,26 @@ int run_make_transfers(vrg_env *env, const float *dirs_local, int32_t k) {
     const size_t words = (size_t)(nleaves + 31) / 32;
     const size_t smem = words <= kBitmapShared ? 4 * words : 0;
     const int64_t scratch_stride = 32 * (int64_t)std::max<size_t>(words, 1) + (words <= kBitmapShared ? 0 : (int64_t)words);
-    // variants, picked per (triangles, rows) bucket: rows walked ray by ray by
-    // 256 or 512 threads, and where they can be traced in tiles (prepare_tiles)
-    // tiles of 128 rays by 512 threads and of 64 by 256 or 128.  On lit rooms of
-    // 420, 816, 2,016 and 8,208 triangles at k = 1,024, 4,096, 8,192 and 65,536
-    // the rows took 1.32, 7.4, 41 and 845 ms walked and 1.11, 5.2, 30.6 and
-    // 423 ms in the best tiles (the widest only at k = 65,536: wider tiles see
-    // more triangles but share them among more rays).
-    using RowKernel = void (*)(DevScene, const LeafInfo *, const FaceRec *, const PatchNode *, const int32_t *,
+    // variants, picked per (triangles, rows) bucket: rows walked ray by ray in
+    // the hierarchy by 256 threads or in the kd tree by 256 or 512, and where
+    // they can be traced in tiles (prepare_tiles) tiles of 128 rays by 512
+    // threads and of 64 by 256 or 128.  On lit rooms of 108, 420, 816, 2,016
+    // and 8,208 triangles at k = 256, 1,024, 4,096, 8,192 and 65,536 the rows took
+    // 0.05, 0.93, 6.4, 42 and 1,605 ms in the hierarchy, 0.07, 1.11, 6.7, 40 and
+    // 845 ms in the kd tree (whose walk suits neighbouring rays) and 0.09, 1.09,
+    // 5.2, 31 and 423 ms in the best tiles (the widest only at k = 65,536: wider
+    // tiles see more triangles but share them among more rays).
+    using RowKernel = void (*)(DevScene, BvhView, const LeafInfo *, const FaceRec *, const PatchNode *, const int32_t *,
                                const int32_t *, const float *, int, int64_t, int64_t, int, int, int, uint32_t *, int64_t,
                                int32_t *, int32_t *, int32_t *);
     using TileKernel = void (*)(DevScene, TileScene, const LeafInfo *, const FaceRec *, const PatchNode *,
                                 const int32_t *, const int32_t *, const float *, int64_t, int64_t, int, int, int,
                                 uint32_t *, int64_t, int32_t *, int32_t *, int32_t *);
-    constexpr int kWalkVariants = 2, kTileVariants = 3;
-    const RowKernel kvar[kWalkVariants] = {k_transfer_rows<256>, k_transfer_rows<512>};
+    constexpr int kWalkVariants = 3, kTileVariants = 3;
+    const RowKernel kvar[kWalkVariants] = {k_transfer_rows<256, true>, k_transfer_rows<256, false>,
+                                            k_transfer_rows<512, false>};
     const TileKernel tvar[kTileVariants] = {k_transfer_tiles<4, 512>, k_transfer_tiles<2, 256>, k_transfer_tiles<2, 128>};
-    const int vthreads[kWalkVariants + kTileVariants] = {256, 512, 512, 256, 128};
+    const int vthreads[kWalkVariants + kTileVariants] = {256, 256, 512, 512, 256, 128};
     const int tbundles[kTileVariants] = {4, 2, 2};
     const size_t tile_smem = smem + 28 * (size_t)ts.nclusters;
     for (const RowKernel kern : kvar)
@@ -1096,9 +1103,9 @@ int run_make_transfers(vrg_env *env, const float *dirs_local, int32_t k) {
                     d_nnz);
             } else {
                 // a row block never has more threads than rays
-                const int vv = vthreads[v] <= k ? v : 0;
+                const int vv = vthreads[v] <= k ? v : v == 2 ? 1 : v;
                 kvar[vv]<<<grid, std::min(vthreads[vv], k), smem, ctx->stream>>>(
-                    s, env->d_leaf_info.as<LeafInfo>(), env->d_faces.as<FaceRec>(),
+                    s, bvh_view(env), env->d_leaf_info.as<LeafInfo>(), env->d_faces.as<FaceRec>(),
                     env->d_patch_nodes.as<PatchNode>(), env->d_face_root.as<int32_t>(),
                     env->d_tri_face.as<int32_t>(), d_dirs, k, r0, nr, nleaves, tsize, limit,
                     counters, scratch_stride, stage_col, stage_cnt,
@@ -1122,7 +1129,7 @@ int run_make_transfers(vrg_env *env, const float *dirs_local, int32_t k) {
         auto sorted_rows = [&](const int64_t *rp) -> cudaError_t {
             timing_begin(ctx, "transfer_rows_sorted", &ev);
             k_transfer_rows_sorted<512><<<ovf_grid, ovf_threads, 0, ctx->stream>>>(
-                s, env->d_leaf_info.as<LeafInfo>(), env->d_faces.as<FaceRec>(), env->d_patch_nodes.as<PatchNode>(),
+                s, bvh_view(env), env->d_leaf_info.as<LeafInfo>(), env->d_faces.as<FaceRec>(), env->d_patch_nodes.as<PatchNode>(),
                 env->d_face_root.as<int32_t>(), env->d_tri_face.as<int32_t>(), d_dirs, k,
                 ovf_rows.as<int64_t>(), novf, ovf_scratch.as<int32_t>(), rp, env->d_col.as<int32_t>(),
                 env->d_weight.as<float>(), ovf_nnz.as<int32_t>());

@@ -80,6 +80,28 @@ __host__ __device__ inline const uint32_t *wall_table(const DevScene &s) {
     return reinterpret_cast<const uint32_t *>(s.leaf_edges + 2 * (s.leaf_edges - s.leaf_planes));
 }
 
+// A node of the line queries' hierarchy (bvhbuild.cpp), half a line: the four
+// children's bounds in steps of a power of two from an origin, one byte each
+// (bound[2 * axis] lower, [2 * axis + 1] upper, child c in byte c; a step or
+// more outside the child's box, which covers the rounding of bvh_step).  A
+// child word is a node index, or kBvhLeafBit | first record << 3 |
+// records - 1; an unused child is inside out.
+constexpr int kBvhLeaf = 4;
+constexpr uint32_t kBvhLeafBit = 1u << 31;
+constexpr uint32_t kBvhNone = 0xffffffffu;
+constexpr int kBvhStack = 64;
+struct alignas(64) BvhNode {
+    float origin[3], step_z;
+    uint32_t bound[6];
+    uint32_t child[4];
+    float step_x, step_y;
+};
+static_assert(sizeof(BvhNode) == 64, "read as four 16-byte words");
+struct BvhView {
+    const float4 *nodes;  // 4 per node; null: the scene has none
+    int64_t base;         // leaf record of the leaves' first triangle
+};
+
 // Sky maps.  The sky-ambient light sends lines in 162 fixed directions, so
 // per direction the scene is a picture seen along parallel lines: points are
 // sheared along the direction onto the plane of the other two axes (cell

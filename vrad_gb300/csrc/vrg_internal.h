@@ -145,7 +145,7 @@ struct vrg_env {
     int32_t wall_tris[6 * vrg::kWallSlots];  // wall slots per scene-box face (-1: unused)
     int32_t wall_counts[6] = {0, 0, 0, 0, 0, 0};
     std::vector<uint32_t> wall_cells;  // the wall-cell table (see vrg_device.h)
-    size_t n_wall_records = 0;          // wall triangles' leaf records after the leaf entries
+    size_t n_extra_records = 0;         // leaf records after the leaf entries: the walls', the hierarchy's
     int wall_layout = 0;                // 0: wall slots, 1: wall cells (see vrg_device.h)
     WalkTreeCosts walk_costs;
     int walk_builder = -1;  // walk tree: 0 host (full sweep), 1 GPU (binned), -1 by size
@@ -157,6 +157,11 @@ struct vrg_env {
     vrg::DevBuf d_nodes, d_leaf_tris, d_tri_ids, d_tri_normals;
     vrg::DevBuf d_top;       // top levels of the tree (kTopNodes entries at most)
     uint32_t ntop = 0;
+    // the line queries' hierarchy: its leaves' triangles in order, their first
+    // leaf record, the nodes
+    std::vector<int32_t> bvh_order;
+    int64_t tri_base = 0, bvh_nodes = 0;
+    vrg::DevBuf d_bvh;
 
     // transparent shadows (coverage.cu): per-triangle flags and coverage
     vrg::DevBuf d_tri_flags, d_tri_cover;
@@ -259,6 +264,7 @@ void scene_bounds(const std::vector<float> &xyz, float *mn, float *mx);
 void build_kd_tree(const std::vector<float> &xyz, HostTree &tree, float *mn, float *mx);
 void build_walk_tree(const std::vector<float> &xyz, const float *mn, const float *mx,
                      const WalkTreeCosts &cost, HostTree &tree);
+void build_bvh(const std::vector<float> &xyz, std::vector<int32_t> &order, std::vector<BvhNode> &nodes);  // bvhbuild.cpp
 int build_walk_tree_device(vrg_env *env, HostTree &tree);  // kdbuild_gpu.cu
 void light_set_falloff(const vrg_light_keys &k, vrg_light &l);
 void light_parse_spot(const vrg_light_keys &k, vrg_light &l);
@@ -266,6 +272,7 @@ int make_rect_patches(const vrg_env &env, float max_chop, float min_chop, PatchS
 
 // device launchers (trace.cu, direct.cu, transfer.cu, bounce.cu)
 DevScene scene_view(const vrg_env *env);
+BvhView bvh_view(const vrg_env *env);
 int launch_occlusion_mask(vrg_env *env, const float *start, const float *stop, int64_t n,
                           int32_t skip_id, uint32_t *mask, int32_t *hit, float *t);
 int launch_trace_closest(vrg_env *env, const float *orig, const float *dir, const float *tmin,

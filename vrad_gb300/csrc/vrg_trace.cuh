@@ -35,7 +35,6 @@ constexpr int32_t kTraceIdSky = 0x01000000;
 // shared memory (stage_top).
 constexpr int kOptStream = 1;
 constexpr int kOptTop = 2;
-constexpr int kOptPipe = 8;    // unit rounds: the next triangle's plane loads during this test
 constexpr int kOptSkip = 16;   // children flagged as leaves without triangles are not visited
 // kOptShRay: the walk constants of each lane's ray are kept in shared memory,
 // one float4 (inv, A, B, neg) per axis and lane, and an inner step reads its
@@ -43,10 +42,6 @@ constexpr int kOptSkip = 16;   // children flagged as leaves without triangles a
 // blocks of at most kShRayLanes threads.
 constexpr int kOptShRay = 32;
 constexpr int kShRayLanes = 128;
-// kOptOneVote (unit-round walks): the idle lanes follow from the busy ballot
-// and a warp-wide mask of the lanes out of work, one ballot per round
-// instead of two.
-constexpr int kOptOneVote = 64;
 // kOptSign: a triangle test gives up before its division when the plane lies
 // behind the origin (the quotient's sign is known).
 constexpr int kOptSign = 128;
