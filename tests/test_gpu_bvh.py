@@ -1,5 +1,6 @@
-"""The line queries' hierarchy against testing every triangle: trees and rays
-at which a bound could be a rounding too tight."""
+"""Line queries against testing every triangle: trees and rays at which a bound
+of the hierarchy could be a rounding too tight (more than 4,096 rays walk it),
+and the same through the kernel that tests every triangle for few rays."""
 import numpy as np
 import pytest
 
@@ -42,7 +43,8 @@ def _soup(kind, rng):
 
 
 @pytest.mark.parametrize("kind", ["plain", "one", "five", "tiny", "far", "flat", "same", "line", "degenerate"])
-def test_queries_equal_brute_force(gpu_ctx, oracle, kind):
+@pytest.mark.parametrize("m", [1, 33, 2500, 6000])
+def test_queries_equal_brute_force(gpu_ctx, oracle, kind, m):
     from vrad_gb300.environment import Environment
 
     rng = np.random.default_rng(17)
@@ -55,7 +57,6 @@ def test_queries_equal_brute_force(gpu_ctx, oracle, kind):
     tri = tri[np.isfinite(tri).all(axis=(1, 2))]
     lo, hi = tri.min(axis=(0, 1)), tri.max(axis=(0, 1))
     size = (hi - lo).max()
-    m = 2500
     a = (lo + rng.uniform(-0.3, 1.3, (m, 3)) * (hi - lo)).astype(np.float32)
     b = (lo + rng.uniform(-0.3, 1.3, (m, 3)) * (hi - lo)).astype(np.float32)
     b[::4] = tri[rng.integers(0, len(tri), len(b[::4]))].mean(axis=1)  # ends on triangles

@@ -110,6 +110,33 @@ const void *pinned_view(const void *p) {
     return a.type == cudaMemoryTypeHost ? a.devicePointer : nullptr;
 }
 
+// A small call's arrays in the context's page-locked memory: inputs are
+// copied there and read by the kernel in place, outputs written there by the
+// kernel (or copied there by the stream) and picked up after the call's one
+// synchronisation.  Each of the pageable copies it stands for cost 5 to 10 us.
+struct Staged {
+    std::unique_lock<std::mutex> lock;
+    char *base = nullptr;
+    size_t at = 0;
+    Staged(vrg_ctx *ctx, size_t bytes) {
+        if (!ctx->stage || bytes + 1024 > kStageBytes) return;
+        lock = std::unique_lock<std::mutex>(ctx->stage_mu);
+        base = ctx->stage;
+    }
+    explicit operator bool() const { return base != nullptr; }
+    template <class T>
+    T *room(int64_t n) {
+        T *p = reinterpret_cast<T *>(base + at);
+        at = (at + sizeof(T) * (size_t)n + 127) & ~(size_t)127;
+        return p;
+    }
+    const float *in(const float *src, int64_t n) {
+        float *p = room<float>(n);
+        memcpy(p, src, sizeof(float) * (size_t)n);
+        return p;
+    }
+};
+
 int download(vrg_ctx *ctx, void *dst, const DevBuf &buf, size_t bytes) {
     if (bytes) VRG_CUDA(ctx, cudaMemcpyAsync(dst, buf.ptr, bytes, cudaMemcpyDeviceToHost, ctx->stream));
     return VRG_OK;
@@ -157,6 +184,14 @@ int vrg_ctx_create(int device, vrg_ctx **out) {
         return e == cudaErrorMemoryAllocation ? VRG_ERR_NOMEM : VRG_ERR_CUDA;
     }
     ctx->stream = ctx->own_stream;
+    // without it (mapped under a unified address space) small calls copy
+    void *stage = nullptr;
+    int unified = 0;
+    if (cudaDeviceGetAttribute(&unified, cudaDevAttrUnifiedAddressing, device) == cudaSuccess && unified &&
+        cudaMallocHost(&stage, kStageBytes) == cudaSuccess)
+        ctx->stage = static_cast<char *>(stage);
+    else
+        (void)cudaGetLastError();
     // the no-alloc bounce's device array and kernels are set up now, so that
     // its calls allocate nothing; a failure here is reported by that call
     if (vrg::noalloc_prepare(ctx) != VRG_OK) ctx->last_error.clear();
@@ -178,6 +213,7 @@ void vrg_ctx_destroy(vrg_ctx *ctx) {
     }
     for (cudaEvent_t e : ctx->event_pool) cudaEventDestroy(e);
     if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
+    if (ctx->stage) cudaFreeHost(ctx->stage);
     delete ctx;
 }
 
@@ -343,6 +379,16 @@ int vrg_env_trace_closest(vrg_env *env, const float *orig, const float *dir, con
     if (n == 0) return VRG_OK;
     std::lock_guard<std::mutex> lk(env->mu);
     vrg_ctx *ctx = env->ctx;
+    if (Staged st(ctx, 40 * (size_t)n); st) {
+        const float *o = st.in(orig, 3 * n), *d = st.in(dir, 3 * n), *t0 = st.in(tmin, n), *t1 = st.in(tmax, n);
+        int32_t *hit = st.room<int32_t>(n);
+        float *t = st.room<float>(n);
+        TRY(launch_trace_closest(env, o, d, t0, t1, n, skip_id, hit, t));
+        TRY(sync(ctx));
+        memcpy(out_hit, hit, 4 * (size_t)n);
+        memcpy(out_t, t, 4 * (size_t)n);
+        return VRG_OK;
+    }
     // page-locked inputs are read in place, others copied first
     const float *d_orig = static_cast<const float *>(pinned_view(orig));
     const float *d_dir = static_cast<const float *>(pinned_view(dir));
@@ -408,6 +454,22 @@ int vrg_env_occlusion_mask(vrg_env *env, const float *start, const float *stop, 
     vrg_ctx *ctx = env->ctx;
     const bool want = out_hit && out_t;
     const int64_t words = (n + 31) / 32;
+    if (Staged st(ctx, 36 * (size_t)n); st) {
+        const float *a = st.in(start, 3 * n), *b = st.in(stop, 3 * n);
+        int32_t *hit = want ? st.room<int32_t>(n) : nullptr;
+        float *t = want ? st.room<float>(n) : nullptr;
+        uint32_t *mask = st.room<uint32_t>(words);
+        VRG_CUDA(ctx, env->d_out2.reserve(4 * words));  // (bits are set by device atomics)
+        TRY(launch_occlusion_mask(env, a, b, n, skip_id, env->d_out2.as<uint32_t>(), hit, t));
+        TRY(download(ctx, mask, env->d_out2, 4 * words));
+        TRY(sync(ctx));
+        memcpy(out_mask, mask, 4 * (size_t)words);
+        if (want) {
+            memcpy(out_hit, hit, 4 * (size_t)n);
+            memcpy(out_t, t, 4 * (size_t)n);
+        }
+        return VRG_OK;
+    }
     // page-locked end points are read where they are (the walk reads each
     // line's 24 bytes once, as it takes the line); others are copied first
     const float *d_start = static_cast<const float *>(pinned_view(start));
@@ -443,6 +505,14 @@ int vrg_env_test_line_does_hit_sky(vrg_env *env, const float *start, const float
     vrg_ctx *ctx = env->ctx;
     // testline.go:36: skip id = TRACE_ID_STATICPROP | staticPropToSkip
     const int32_t skip = VRG_TRACE_ID_STATICPROP | static_prop_to_skip;
+    if (Staged st(ctx, 28 * (size_t)n); st) {
+        const float *a = st.in(start, 3 * n), *b = st.in(stop, 3 * n);
+        float *frac = st.room<float>(n);
+        TRY(launch_test_lines(env, a, b, n, skip, frac));
+        TRY(sync(ctx));
+        memcpy(fraction_visible, frac, 4 * (size_t)n);
+        return VRG_OK;
+    }
     const float *d_start = static_cast<const float *>(pinned_view(start));
     const float *d_stop = static_cast<const float *>(pinned_view(stop));
     if (!d_start || !d_stop) {

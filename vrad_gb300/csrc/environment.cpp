@@ -382,6 +382,9 @@ int vrg_env_setup_acceleration_structure(vrg_env *env) {
     env->cover_ready = false;
     if (ctx->host_only) return VRG_OK;
     VRG_CUDA(ctx, cudaSetDevice(ctx->device));
+    VRG_CUDA(ctx, env->d_few.reserve(kFewBytes));
+    VRG_CUDA(ctx, cudaMemsetAsync(env->d_few.ptr, 0xff, kFewKeyBytes, ctx->stream));
+    VRG_CUDA(ctx, cudaMemsetAsync(env->d_few.as<char>() + kFewKeyBytes, 0, kFewBytes - kFewKeyBytes, ctx->stream));
     if (!bvh.empty()) {
         VRG_CUDA(ctx, env->d_bvh.reserve(bvh.size() * sizeof(BvhNode)));
         VRG_CUDA(ctx, cudaMemcpyAsync(env->d_bvh.ptr, bvh.data(), bvh.size() * sizeof(BvhNode), cudaMemcpyHostToDevice,

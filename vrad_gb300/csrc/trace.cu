@@ -1,6 +1,8 @@
 // trace.cu -- batched ray queries against a resident scene (Trace4Rays,
 // raytracer/environment.go:140-145, and TestLineDoesHitSky,
 // raytracer/trace/testline.go:18-94).
+#include <algorithm>
+
 #include "vrg_internal.h"
 #include "vrg_bvh.cuh"
 #include "vrg_trace.cuh"
@@ -144,6 +146,156 @@ __global__ void __launch_bounds__(kThreads, MINB) k_bvh(DevScene s, BvhView bv, 
     }
 }
 
+// Few rays: every triangle is tested, 32 rays to a block and the triangles
+// split over blockIdx.y and the block's warps.  A walk is a chain of dependent
+// loads whatever the number of rays (23 us for four rays among 12,300
+// triangles, 37 for 33); testing all of them keeps the whole GPU busy (10 and
+// 12 us) until the tests cost more: about 4 us a million, a lane of the 32 or
+// other taking the whole test nearly every time.  Each block takes the least
+// (t, index) of its share per ray; blocks of one group of rays meet in `keys`,
+// and the last one to finish writes the answers and leaves keys and counters
+// as it found them.  The answer is the walk's: both are what testing every
+// triangle gives.
+constexpr int kFewWarps = 4, kFewUnroll = 4;
+constexpr unsigned long long kFewNone = ~0ull;
+
+template <Query Q>
+__global__ void __launch_bounds__(32 * kFewWarps) k_few(DevScene s, QueryArgs q, int64_t base, int ntris, int slices,
+                                                        unsigned long long *__restrict__ keys,
+                                                        unsigned int *__restrict__ done) {
+    __shared__ unsigned long long least[kFewWarps][32];
+    __shared__ bool last_sh;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int64_t i = (int64_t)blockIdx.x * 32 + lane;
+    Ray ray{0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+    float t0 = 0.0f, t1 = -1.0f;
+    if (i < q.n) {
+        if (Q == kQClosest) {
+            load3(q.a, i, ray.ox, ray.oy, ray.oz);
+            load3(q.b, i, ray.dx, ray.dy, ray.dz);
+            t0 = __ldg(q.tmin + i);
+            t1 = __ldg(q.tmax + i);
+        } else {
+            float sx, sy, sz, ex, ey, ez;
+            load3(q.a, i, sx, sy, sz);
+            load3(q.b, i, ex, ey, ez);
+            const Line L = make_line(sx, sy, sz, ex, ey, ez);
+            ray = Ray{L.ox, L.oy, L.oz, L.dx, L.dy, L.dz};
+            t1 = L.len;  // zero length: nothing in [0, 0)
+        }
+    }
+    // this warp's triangles: first, first + kFewWarps, ... < end
+    const int share = (ntris + slices - 1) / slices;
+    const int first = blockIdx.y * share + wid, end = min(ntris, ((int)blockIdx.y + 1) * share);
+    const float4 *planes = s.leaf_planes + base, *edges = s.leaf_edges + 2 * base;
+    int32_t best = -1;
+    float best_t = t1;  // the first hit must be below
+    for (int k0 = first; k0 < end; k0 += kFewWarps * kFewUnroll) {
+        float4 w0[kFewUnroll];
+#pragma unroll
+        for (int u = 0; u < kFewUnroll; u++) {
+            const int k = k0 + kFewWarps * u;
+            w0[u] = k < end ? __ldg(planes + k) : make_float4(0.0f, 0.0f, 0.0f, __int_as_float(0x7fc00000));
+        }
+#pragma unroll
+        for (int u = 0; u < kFewUnroll; u++) {
+            const int k = k0 + kFewWarps * u;
+            const float den = dot3r(w0[u].x, w0[u].y, w0[u].z, ray.dx, ray.dy, ray.dz);
+            const float num = rsub(w0[u].w, dot3r(w0[u].x, w0[u].y, w0[u].z, ray.ox, ray.oy, ray.oz));
+            // t < 0 where that is out of range, or past the best hit by more
+            // than the quotient's rounding
+            const bool neg = ((__float_as_uint(num) ^ __float_as_uint(den)) >> 31) != 0u;
+            if (neg ? t0 >= 0.0f && fabsf(num) > 1e-30f : fabsf(num) > best_t * fabsf(den) * 1.000001f) continue;
+            const float t = rdiv(num, den);
+            if (!(t >= t0 && t < t1 && t <= best_t)) continue;
+            const float4 w2 = __ldg(edges + 2 * (size_t)k + 1);
+            if (__float_as_int(w2.z) == q.skip) continue;
+            const float4 w1 = __ldg(edges + 2 * (size_t)k);
+            const int drop = (int)(__float_as_uint(w2.w) & 3u);
+            const float h0 = radd(pick3(drop, ray.oy, ray.oz, ray.ox), rmul(t, pick3(drop, ray.dy, ray.dz, ray.dx)));
+            const float h1 = radd(pick3(drop, ray.oz, ray.ox, ray.oy), rmul(t, pick3(drop, ray.dz, ray.dx, ray.dy)));
+            const float b0 = radd(radd(rmul(w1.x, h0), rmul(w1.z, h1)), w2.x);
+            const float b1 = radd(radd(rmul(w1.y, h0), rmul(w1.w, h1)), w2.y);
+            if (b0 >= 0.0f && b1 >= 0.0f && rsub(rsub(1.0f, b0), b1) >= 0.0f) {
+                const int32_t ti = (int32_t)(__float_as_uint(w2.w) >> 2);
+                if (t < best_t || best < 0 || ti < best) {
+                    best = ti;
+                    best_t = t;
+                }
+            }
+        }
+    }
+    // (t, index) as one number that orders the same (-0 as +0, its sign in the
+    // last bit)
+    unsigned long long key = kFewNone;
+    if (best >= 0) {
+        const uint32_t u = __float_as_uint(best_t + 0.0f);
+        key = ((unsigned long long)(u ^ ((u >> 31) ? 0xffffffffu : 0x80000000u)) << 32) | ((uint32_t)best << 1) |
+              (best_t == 0.0f && signbit(best_t) ? 1u : 0u);
+    }
+    least[wid][lane] = key;
+    __syncthreads();
+    if (wid != 0) return;
+#pragma unroll
+    for (int w = 1; w < kFewWarps; w++) key = min(key, least[w][lane]);
+    if (slices > 1) {
+        if (i < q.n && key != kFewNone) atomicMin(keys + i, key);
+        __threadfence();
+        __syncwarp();
+        if (lane == 0) last_sh = atomicAdd(done + blockIdx.x, 1u) == (unsigned)slices - 1u;
+        __syncwarp();
+        if (!last_sh) return;
+        __threadfence();
+        if (i < q.n) key = atomicExch(keys + i, kFewNone);
+        if (lane == 0) done[blockIdx.x] = 0u;
+    }
+    best = -1;
+    best_t = kInf;
+    bool occ = false;
+    if (key != kFewNone) {
+        best = (int32_t)((uint32_t)key >> 1);
+        const uint32_t u = (uint32_t)(key >> 32);
+        best_t = (key & 1u) ? -0.0f : __uint_as_float(u ^ ((u >> 31) ? 0x80000000u : 0xffffffffu));
+        occ = (__ldg(&s.tri_ids[best]) & kTraceIdSky) == 0;
+    }
+    if (Q == kQMask || Q == kQMaskHit) {
+        const unsigned word = __ballot_sync(0xffffffffu, i < q.n && occ);
+        if (lane == 0) q.mask[blockIdx.x] = word;
+    }
+    if (i < q.n) {
+        if (Q == kQLines) q.frac[i] = occ ? 0.0f : 1.0f;
+        if (Q == kQClosest || Q == kQMaskHit) {
+            q.hit[i] = best;
+            q.t[i] = best_t;
+        }
+    }
+}
+
+// Whether n rays are few enough against the scene for k_few, at 9 us and 4 us
+// more a million tests.  The hierarchy takes 12 us for 33 to 1,000 rays among
+// 204 triangles, 23 among 2,064, 37 to 40 among 12,300, 55 to 60 among 49,164.
+bool few_rays(const vrg_env *env, int64_t n) {
+    const int64_t rays = (n + 31) & ~(int64_t)31, tris = (int64_t)env->bvh_order.size();
+    return n <= kFewRays && tris > 0 && rays * tris <= (tris >= 8192 ? 6000000 : 3000000) && env->d_few.ptr;
+}
+
+template <Query Q>
+cudaError_t launch_few(vrg_env *env, const char *name, const QueryArgs &q) {
+    vrg_ctx *ctx = env->ctx;
+    const int groups = (int)((q.n + 31) / 32), tris = (int)env->bvh_order.size();
+    // enough blocks for the GPU, at least four triangles to a warp
+    const int64_t want = ((int64_t)ctx->num_sms * 8 + groups - 1) / groups;
+    const int slices = (int)std::max<int64_t>(1, std::min<int64_t>(want, tris / (kFewWarps * kFewUnroll)));
+    cudaEvent_t ev = nullptr;
+    timing_begin(ctx, name, &ev);
+    k_few<Q><<<dim3(groups, slices), 32 * kFewWarps, 0, ctx->stream>>>(
+        scene_view(env), q, env->tri_base, tris, slices, env->d_few.as<unsigned long long>(),
+        reinterpret_cast<unsigned int *>(env->d_few.as<char>() + kFewKeyBytes));
+    const cudaError_t e = cudaGetLastError();
+    timing_end(ctx, name, ev);
+    return e;
+}
+
 // Persistent grid: resident blocks per SM times SMs, but no more blocks
 // than the rays can keep busy.
 template <class K>
@@ -162,6 +314,7 @@ int persistent_grid(const vrg_ctx *ctx, K kernel, int64_t n) {
 template <Query Q, bool ORDER>
 cudaError_t launch_query(vrg_env *env, const char *name, QueryArgs q) {
     vrg_ctx *ctx = env->ctx;
+    if (few_rays(env, q.n)) return launch_few<Q>(env, name, q);
     const auto kernel = k_bvh<Q, 4, 4, 8, 8, ORDER>;
     cudaError_t e = env->d_work.reserve(256);
     if (e != cudaSuccess) return e;

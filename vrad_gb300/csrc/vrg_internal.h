@@ -60,6 +60,14 @@ struct BounceGraph;   // bounce.cu: the scene's bounce loop as a graph
 
 constexpr size_t kScratchKept = (size_t)256 << 20;
 
+// k_few (trace.cu): queries of at most this many rays, a 64-bit key each, and
+// a counter per 32.
+constexpr int64_t kFewRays = 4096;
+constexpr size_t kFewKeyBytes = 8 * kFewRays, kFewBytes = kFewKeyBytes + 4 * (kFewRays / 32);
+// Page-locked host memory of a context through which small host-buffer calls
+// pass their arrays.
+constexpr size_t kStageBytes = (size_t)1 << 20;
+
 struct KernelStat {
     double ms = 0.0;
     int64_t launches = 0;
@@ -88,6 +96,10 @@ struct vrg_ctx {
     bool autotune = true;
     uint64_t hbm_reserve = (uint64_t)1 << 30;  // kept free when admitting a relight scene
     int32_t xfer_table_limit = 7168;            // distinct targets per transfer row held in shared memory
+    // kStageBytes of page-locked memory that kernels read and write in place
+    // (null: not to be had), one call at a time
+    std::mutex stage_mu;
+    char *stage = nullptr;
     // scratch of the sky-map and transfer builds, which hold scratch_mu until
     // their kernels are done; at most kScratchKept of it is kept between them
     std::mutex scratch_mu;
@@ -157,6 +169,7 @@ struct vrg_env {
     vrg::DevBuf d_nodes, d_leaf_tris, d_tri_ids, d_tri_normals;
     vrg::DevBuf d_top;       // top levels of the tree (kTopNodes entries at most)
     uint32_t ntop = 0;
+    vrg::DevBuf d_few;       // k_few's least hits and block counters, as it leaves them (kFewBytes)
     // the line queries' hierarchy: its leaves' triangles in order, their first
     // leaf record, the nodes
     std::vector<int32_t> bvh_order;

@@ -40,7 +40,7 @@ class LightKeys(C.Structure):
 
 
 def _p(a):
-    return None if a is None else C.c_void_p(a.ctypes.data)
+    return None if a is None else a.__array_interface__["data"][0]
 
 
 def _f32(a, shape=None):
