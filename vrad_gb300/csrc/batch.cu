@@ -25,6 +25,7 @@ namespace {
 
 constexpr int kThreads = 128;
 static_assert(kThreads <= kShRayLanes, "kOptShRay keeps one slot per thread of a block");
+static_assert(kThreads <= 32 * kSkyWarps, "sky_fraction keeps one slot per warp of a block");
 constexpr int kSpmvThreads = 256;
 constexpr int kGraphBounces = 8;
 
@@ -65,7 +66,8 @@ __device__ __forceinline__ int upper_segment(const int64_t *__restrict__ start, 
 }
 
 // Work items: segments [0, E) are scene e's luxel supersamples (ss per
-// luxel, in luxel order), segments [E, 2E) scene e's leaf-patch points.
+// luxel, in luxel order), segments [E, 2E) scene e's leaf-patch points, each
+// rounded up to a whole warp of items.
 // OPT: walk options (kOptShRay or none); MINB: resident blocks per SM.
 template <bool MAP, int OPT, int MINB>
 __global__ void __launch_bounds__(kThreads, MINB) k_batch_gather(
@@ -84,10 +86,13 @@ __global__ void __launch_bounds__(kThreads, MINB) k_batch_gather(
         bool luxel_item = false;
         int64_t lux = 0;
         float *lux_out = nullptr;
-        if (gi < total) {
-            const int sg = upper_segment(seg, 2 * nscenes, gi);
-            const int64_t local = gi - __ldg(seg + sg);
-            const BatchDesc *d = descs + (sg < nscenes ? sg : sg - nscenes);
+        // segments start at multiples of 32: the warp's items are of one
+        const int sg = upper_segment(seg, 2 * nscenes, (int64_t)wb);
+        const BatchDesc *d = descs + (sg < nscenes ? sg : sg - nscenes);
+        const int64_t local = gi - __ldg(seg + sg);
+        const bool have = local < (sg < nscenes ? d->nlux * ss : d->npts);
+        const unsigned lanes = __ballot_sync(0xffffffffu, have);
+        if (have) {
             // the item's point and normal, then one gather_point call site
             // (a second inlined copy of the gather costs through code size)
             float px, py, pz, nx, ny, nz;
@@ -114,7 +119,7 @@ __global__ void __launch_bounds__(kThreads, MINB) k_batch_gather(
                 ny = __ldg(n + 1);
                 nz = __ldg(n + 2);
             }
-            gather_point<kSkyTrace, OPT, kWallAny, MAP>(d->scene, d->sky, d->lights, d->nl, px, py, pz, nx, ny, nz, r, g, b, rays);
+            gather_point<kSkyTrace, OPT, kWallAny, MAP>(d->scene, d->sky, lanes, d->lights, d->nl, px, py, pz, nx, ny, nz, r, g, b, rays);
             if (!luxel_item) {
                 float *o = d->pout + 3 * local;
                 o[0] = r;
@@ -123,8 +128,7 @@ __global__ void __launch_bounds__(kThreads, MINB) k_batch_gather(
             }
         }
         if (ss == 4) {
-            // luxel segments start at multiples of 4, so a luxel's samples
-            // are the four lanes of one aligned quad
+            // a luxel's samples are the four lanes of one aligned quad
             const float r1 = __shfl_down_sync(0xffffffffu, r, 1), r2 = __shfl_down_sync(0xffffffffu, r, 2),
                         r3 = __shfl_down_sync(0xffffffffu, r, 3);
             const float g1 = __shfl_down_sync(0xffffffffu, g, 1), g2 = __shfl_down_sync(0xffffffffu, g, 2),
@@ -361,13 +365,14 @@ int vrg_batch_bake(vrg_batch *b, int32_t supersamples, uint64_t seed, int32_t ma
     bool map = true;
     for (int e = 0; e < E; e++) map = use_sky_map(b->envs[e], points[e], all_points >= repay) && map;
     std::vector<BatchDesc> descs(E);
+    const auto whole_warps = [](int64_t n) { return (n + 31) & ~(int64_t)31; };
     std::vector<int64_t> seg(2 * E + 1, 0), rstart(E + 1, 0);
     for (int e = 0; e < E; e++) {
         descs[e] = make_desc(b->envs[e]);
-        seg[e + 1] = seg[e] + descs[e].nlux * supersamples;
+        seg[e + 1] = seg[e] + whole_warps(descs[e].nlux * supersamples);
         rstart[e + 1] = rstart[e] + descs[e].rows;
     }
-    for (int e = 0; e < E; e++) seg[E + e + 1] = seg[E + e] + descs[e].npts;
+    for (int e = 0; e < E; e++) seg[E + e + 1] = seg[E + e] + whole_warps(descs[e].npts);
     const int64_t rows = rstart[E];
     VRG_CUDA(ctx, b->d_desc.reserve(sizeof(BatchDesc) * E));
     VRG_CUDA(ctx, b->d_seg.reserve(8 * seg.size()));

@@ -17,6 +17,7 @@ namespace {
 
 constexpr int kThreads = 128;
 static_assert(kThreads <= kShRayLanes, "kOptShRay keeps one slot per thread of a block");
+static_assert(kThreads <= 32 * kSkyWarps, "sky_fraction keeps one slot per warp of a block");
 
 
 // One thread per supersample; the S = 4 samples of a luxel sit in four
@@ -85,7 +86,8 @@ __global__ void __launch_bounds__(kThreads, MINB) k_direct_luxels(
             ny = fr.normal.y;
             nz = fr.normal.z;
         }
-        if (gi < total) gather_point<kSkyTrace, OPT, WM, MAP>(s, sv, lights, nl, px, py, pz, nx, ny, nz, r, g, b, rays);
+        const unsigned lanes = __ballot_sync(0xffffffffu, gi < total);
+        if (gi < total) gather_point<kSkyTrace, OPT, WM, MAP>(s, sv, lanes, lights, nl, px, py, pz, nx, ny, nz, r, g, b, rays);
         if (is_pt) {
             const int64_t i = gi - nsamp;
             pout[3 * i] = r;
@@ -123,9 +125,10 @@ __global__ void __launch_bounds__(kThreads, 8) k_direct_points(
     uint32_t rays = 0;
     for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < n; base += stride) {
         const int64_t i = base + threadIdx.x;
+        const unsigned lanes = __ballot_sync(0xffffffffu, i < n);
         if (i < n) {
             float r, g, b;
-            gather_point<kSkyTrace, 0, kWallAny, MAP>(s, sv, lights, nl, __ldg(pts + 3 * i), __ldg(pts + 3 * i + 1), __ldg(pts + 3 * i + 2),
+            gather_point<kSkyTrace, 0, kWallAny, MAP>(s, sv, lanes, lights, nl, __ldg(pts + 3 * i), __ldg(pts + 3 * i + 1), __ldg(pts + 3 * i + 2),
                          __ldg(nrm + 3 * i), __ldg(nrm + 3 * i + 1), __ldg(nrm + 3 * i + 2), r, g, b, rays);
             out[3 * i] = r;
             out[3 * i + 1] = g;

@@ -37,6 +37,7 @@ namespace vrg {
 namespace {
 
 constexpr int kThreads = 128;
+static_assert(kThreads <= 32 * kSkyWarps, "sky_fraction keeps one slot per warp of a block");
 constexpr int kSpmvThreads = 256;
 constexpr int kRelightMaxBlocks = 2048;  // SpMV grid cap of a relight (partials slots)
 
@@ -96,7 +97,10 @@ __global__ void __launch_bounds__(kThreads, 8) k_relight_gather(
         const int64_t gi = (int64_t)wb + lane;
         float r = 0.0f, g = 0.0f, b = 0.0f;
         bool luxel_item = false;
-        int64_t lux = 0;
+        int64_t lux = 0, leaf = 0;
+        float px = 0.0f, py = 0.0f, pz = 0.0f, nx = 0.0f, ny = 0.0f, nz = 0.0f;
+        float *sky = nullptr;
+        uint32_t *vis = nullptr;
         if (gi < nsamp) {
             luxel_item = true;
             int f;
@@ -117,13 +121,14 @@ __global__ void __launch_bounds__(kThreads, 8) k_relight_gather(
             tile_luxel(lux - __ldg(luxel_off + f), fr.nu, fr.nv, iu, iv);
             lux = __ldg(luxel_off + f) + (int64_t)iv * fr.nu + iu;
             const int64_t gsamp = lux * ss + kk;
-            float px, py, pz;
             luxel_sample(fr, lux, iu, iv, kk, ss, seed, px, py, pz);
-            gather_point<SKY, 0, kWallAny, MAP>(s, sv, lights, nl, px, py, pz, fr.normal.x, fr.normal.y, fr.normal.z, r, g,
-                              b, rays, sky_lux + gsamp * sky_slots, vis_lux + gsamp * vis_words, edited);
+            nx = fr.normal.x;
+            ny = fr.normal.y;
+            nz = fr.normal.z;
+            sky = sky_lux + gsamp * sky_slots;
+            vis = vis_lux + gsamp * vis_words;
         } else if (gi < total) {
             const int64_t li = gi - nsamp;
-            int64_t leaf;
             if (all) {
                 leaf = li;
             } else {
@@ -131,9 +136,20 @@ __global__ void __launch_bounds__(kThreads, 8) k_relight_gather(
                 leaf = __ldg(list.leaf_beg + k) + (li - __ldg(list.leaf_off + k));
             }
             const float *p = ppts + 3 * leaf, *n = pnrm + 3 * leaf;
-            gather_point<SKY, 0, kWallAny, MAP>(s, sv, lights, nl, __ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(n), __ldg(n + 1),
-                              __ldg(n + 2), r, g, b, rays, sky_pts + leaf * sky_slots,
-                              vis_pts + leaf * vis_words, edited);
+            px = __ldg(p);
+            py = __ldg(p + 1);
+            pz = __ldg(p + 2);
+            nx = __ldg(n);
+            ny = __ldg(n + 1);
+            nz = __ldg(n + 2);
+            sky = sky_pts + leaf * sky_slots;
+            vis = vis_pts + leaf * vis_words;
+        }
+        const unsigned lanes = __ballot_sync(0xffffffffu, gi < total);
+        if (gi < total)
+            gather_point<SKY, 0, kWallAny, MAP>(s, sv, lanes, lights, nl, px, py, pz, nx, ny, nz, r, g, b, rays, sky,
+                                                vis, edited);
+        if (gi < total && !luxel_item) {
             pout[3 * leaf] = r;
             pout[3 * leaf + 1] = g;
             pout[3 * leaf + 2] = b;

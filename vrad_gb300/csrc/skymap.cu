@@ -440,13 +440,14 @@ int build(vrg_env *env, int n) {
     }
     std::vector<SkyDir> dirs;
     make_dirs(env, n, dirs);
-    std::vector<float4> view(3 * kNumAnorms);
+    std::vector<float4> view(4 * kNumAnorms);
     for (int j = 0; j < kNumAnorms; j++) {
-        view[3 * j] = dirs[j].gu;
-        view[3 * j].w -= 0.5f;  // the lookup rounds to the nearest cell
-        view[3 * j + 1] = dirs[j].gv;
-        view[3 * j + 1].w -= 0.5f;
-        view[3 * j + 2] = dirs[j].gd;
+        view[4 * j] = dirs[j].gu;
+        view[4 * j].w -= 0.5f;  // the lookup rounds to the nearest cell
+        view[4 * j + 1] = dirs[j].gv;
+        view[4 * j + 1].w -= 0.5f;
+        view[4 * j + 2] = dirs[j].gd;
+        view[4 * j + 3] = make_float4(dirs[j].d[0], dirs[j].d[1], dirs[j].d[2], 0.0f);
     }
     const bool has_sky = nsky > 0;
     const int64_t pairs = nt * kNumAnorms;
@@ -534,7 +535,7 @@ SkyView sky_view(const vrg_env *env) {
     if (env->sky_n <= 0) return v;
     const size_t cells = (size_t)kNumAnorms * env->sky_n * env->sky_n;
     char *base = env->d_sky_cells.as<char>();
-    const size_t vbytes = 3 * kNumAnorms * sizeof(float4);
+    const size_t vbytes = 4 * kNumAnorms * sizeof(float4);
     v.dirs = reinterpret_cast<const float4 *>(base);
     v.info = reinterpret_cast<const uint2 *>(base + vbytes);
     v.bound = reinterpret_cast<const uint32_t *>(base + vbytes + 8 * cells);

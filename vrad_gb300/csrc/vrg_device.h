@@ -124,7 +124,8 @@ struct SkyView {
     const uint2 *info;      // first pool entry, entries | kSkyCellFlag
     const uint2 *pool;      // leaf-record index, depth above which the triangle is clear; per cell
                             // in descending order of that depth
-    const float4 *dirs;     // per direction: cu, cv and depth as dot products (xyz . p + w)
+    const float4 *dirs;     // per direction: cu, cv and depth as dot products (xyz . p + w), and
+                            // the direction itself
     int32_t n;              // cells per axis
 };
 constexpr uint32_t kSkyPast = 1u << 31;      // in `bound`
