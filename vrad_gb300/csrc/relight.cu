@@ -303,15 +303,15 @@ __global__ void k_digest_partial(const float *__restrict__ lux, int64_t nlux3, c
     }
 }
 
-__global__ void k_digest_final(const double *__restrict__ partials, int nblocks, double *__restrict__ out) {
-    if (threadIdx.x == 0) {
-        double a = 0.0, c = 0.0;
-        for (int i = 0; i < nblocks; i++) {
-            a += partials[2 * i];
-            c += partials[2 * i + 1];
-        }
-        out[0] = a;
-        out[1] = c;
+// (one thread that also loads them, one after another, took 9.4 us)
+__global__ void k_digest_final(const double *__restrict__ partials, double *__restrict__ out) {
+    __shared__ double part[2 * kDigestBlocks];
+    part[threadIdx.x] = partials[threadIdx.x];
+    __syncthreads();
+    if (threadIdx.x < 2) {
+        double a = 0.0;
+        for (int i = 0; i < kDigestBlocks; i++) a += part[2 * i + threadIdx.x];
+        out[threadIdx.x] = a;
     }
 }
 
@@ -346,33 +346,43 @@ int spmv_blocks(const vrg_ctx *ctx) {
 }  // namespace
 
 // Per-slot device scratch of a relight request.
+// What a request of nf faces uploads, in one copy (seven cost 2 us each):
+// the work and ray counters (zero), offsets, face list, edited mask.
+struct RequestBlock {
+    unsigned long long *counters;
+    int64_t *samp_off, *leaf_off;
+    int32_t *faces, *leaf_beg;
+    uint32_t *edited;
+    RequestBlock(char *p, size_t nf) {
+        counters = reinterpret_cast<unsigned long long *>(p);
+        samp_off = reinterpret_cast<int64_t *>(counters + 2);
+        leaf_off = samp_off + (nf + 1);
+        faces = reinterpret_cast<int32_t *>(leaf_off + (nf + 1));
+        leaf_beg = faces + (nf + 1);
+        edited = reinterpret_cast<uint32_t *>(leaf_beg + (nf + 1));
+    }
+    static size_t bytes(size_t nf, size_t nwords) { return 16 + (nf + 1) * (8 + 8 + 4 + 4) + 4 * nwords; }
+};
+
 struct RelightScratch {
-    DevBuf buf;  // [unused | counters | digest | digest partials | offsets | face list | edited mask]
+    DevBuf buf;  // [digest | digest partials | a request: see RequestBlock]
     size_t cap_faces = 0, cap_words = 0;
-    unsigned long long *work = nullptr, *rays = nullptr;
     double *digest = nullptr, *partials = nullptr;
-    int32_t *faces = nullptr, *leaf_beg = nullptr;
-    int64_t *samp_off = nullptr, *leaf_off = nullptr;
-    uint32_t *edited = nullptr;
+    char *request = nullptr;
+    unsigned long long *rays = nullptr;  // the request's shadow-ray counter
 
     int reserve(vrg_ctx *ctx, size_t nfaces, size_t nwords) {
         if (nfaces <= cap_faces && nwords <= cap_words && buf.ptr) return VRG_OK;
         nfaces = std::max(nfaces, cap_faces);
         nwords = std::max(nwords, cap_words);
         const size_t head = 256 + 2 * 8 * kRelightMaxBlocks;
-        const size_t bytes = head + (nfaces + 1) * (4 + 4 + 8 + 8) + 4 * nwords + 256;
+        const size_t bytes = head + RequestBlock::bytes(nfaces, nwords) + 256;
         VRG_CUDA(ctx, buf.reserve(bytes));
         char *p = buf.as<char>();
-        work = reinterpret_cast<unsigned long long *>(p + 64);
-        rays = work + 1;
         digest = reinterpret_cast<double *>(p + 128);
         partials = reinterpret_cast<double *>(p + 256);
-        char *q = p + head;
-        samp_off = reinterpret_cast<int64_t *>(q);
-        leaf_off = samp_off + (nfaces + 1);
-        faces = reinterpret_cast<int32_t *>(leaf_off + (nfaces + 1));
-        leaf_beg = faces + (nfaces + 1);
-        edited = reinterpret_cast<uint32_t *>(leaf_beg + (nfaces + 1));
+        request = p + head;
+        rays = RequestBlock(request, 0).counters + 1;
         cap_faces = nfaces;
         cap_words = nwords;
         return VRG_OK;
@@ -693,30 +703,29 @@ int loop_graph(vrg_env *env, cudaStream_t st, int sblocks, cudaGraphExec_t *out)
 }
 
 // Issues one relight on `st`: table upload, partial re-gather, warm bounce,
-// digest.  Nothing here waits on the GPU.
+// and the digest that only a served request reports.  Nothing here waits on
+// the GPU.
 int issue_relight(vrg_env *env, const RelightPlan &p, int32_t max_iters, float tol, cudaStream_t st,
-                  RelightScratch &sc, HostStage &stage) {
+                  RelightScratch &sc, HostStage &stage, bool digest) {
     vrg_ctx *ctx = env->ctx;
     const int32_t F = env->nfaces;
     const int32_t nf = p.all ? F : (int32_t)p.faces.size();
     int rc = sc.reserve(ctx, (size_t)std::max(nf, 1), p.edited.size());
     if (rc != VRG_OK) return rc;
-    // host staging: light table, then the face list and offsets
+    // host staging: light table, then the request
     const size_t lbytes = 80 * p.table.size();
-    const size_t ebytes = 4 * p.edited.size();
-    const size_t fbytes = (size_t)(nf + 1) * (8 + 8 + 4 + 4);
-    rc = stage.reserve(ctx, lbytes + ebytes + fbytes + 64);
+    const size_t rbytes = RequestBlock::bytes(nf, p.edited.size());
+    rc = stage.reserve(ctx, lbytes + rbytes);
     if (rc != VRG_OK) return rc;
     std::vector<float4> packed;
     pack_lights(p.table, packed);
     char *h = static_cast<char *>(stage.ptr);
     memcpy(h, packed.data(), lbytes);
-    uint32_t *he = reinterpret_cast<uint32_t *>(h + lbytes);
-    memcpy(he, p.edited.data(), ebytes);
-    int64_t *hs = reinterpret_cast<int64_t *>(h + ((lbytes + ebytes + 7) & ~(size_t)7));
-    int64_t *hl = hs + (nf + 1);
-    int32_t *hf = reinterpret_cast<int32_t *>(hl + (nf + 1));
-    int32_t *hb = hf + (nf + 1);
+    const RequestBlock host(h + lbytes, nf), dev(sc.request, nf);
+    host.counters[0] = host.counters[1] = 0;
+    memcpy(host.edited, p.edited.data(), 4 * p.edited.size());
+    int64_t *hs = host.samp_off, *hl = host.leaf_off;
+    int32_t *hf = host.faces, *hb = host.leaf_beg;
     const int ss = env->relight_ss;
     hs[0] = hl[0] = 0;
     for (int32_t k = 0; k < nf; k++) {
@@ -727,13 +736,8 @@ int issue_relight(vrg_env *env, const RelightPlan &p, int32_t max_iters, float t
         hl[k + 1] = hl[k] + (env->face_leaf_begin[2 * f + 1] - env->face_leaf_begin[2 * f]);
     }
     VRG_CUDA(ctx, cudaMemcpyAsync(env->d_lights.ptr, h, lbytes, cudaMemcpyHostToDevice, st));
-    VRG_CUDA(ctx, cudaMemcpyAsync(sc.edited, he, ebytes, cudaMemcpyHostToDevice, st));
-    VRG_CUDA(ctx, cudaMemcpyAsync(sc.samp_off, hs, 8 * (size_t)(nf + 1), cudaMemcpyHostToDevice, st));
-    VRG_CUDA(ctx, cudaMemcpyAsync(sc.leaf_off, hl, 8 * (size_t)(nf + 1), cudaMemcpyHostToDevice, st));
-    VRG_CUDA(ctx, cudaMemcpyAsync(sc.faces, hf, 4 * (size_t)(nf + 1), cudaMemcpyHostToDevice, st));
-    VRG_CUDA(ctx, cudaMemcpyAsync(sc.leaf_beg, hb, 4 * (size_t)(nf + 1), cudaMemcpyHostToDevice, st));
-    VRG_CUDA(ctx, cudaMemsetAsync(sc.work, 0, 16, st));
-    RelightList list{sc.faces, sc.samp_off, sc.leaf_off, sc.leaf_beg, nf};
+    VRG_CUDA(ctx, cudaMemcpyAsync(sc.request, h + lbytes, rbytes, cudaMemcpyHostToDevice, st));
+    RelightList list{dev.faces, dev.samp_off, dev.leaf_off, dev.leaf_beg, nf};
     const int64_t items = hs[nf] + hl[nf];
     if (items > 0) {
         k_relight_gather<kSkyRead><<<persistent_blocks(ctx, (const void *)k_relight_gather<kSkyRead>, items), kThreads, 0, st>>>(
@@ -741,7 +745,7 @@ int issue_relight(vrg_env *env, const RelightPlan &p, int32_t max_iters, float t
             env->d_luxel_offset.as<int64_t>(), F, list, ss, env->relight_seed, env->d_bake_rgb.as<float>(),
             env->d_patch_pts.as<float>(), env->d_patch_nrm.as<float>(), env->d_leaf_direct.as<float>(),
             env->d_sky_lux.as<float>(), env->d_sky_pts.as<float>(), env->sky_slots,
-            env->d_vis_lux.as<uint32_t>(), env->d_vis_pts.as<uint32_t>(), env->vis_words, sc.edited, sc.work,
+            env->d_vis_lux.as<uint32_t>(), env->d_vis_pts.as<uint32_t>(), env->vis_words, dev.edited, dev.counters,
             sc.rays);
         VRG_CUDA(ctx, cudaGetLastError());
     }
@@ -760,13 +764,15 @@ int issue_relight(vrg_env *env, const RelightPlan &p, int32_t max_iters, float t
     rc = loop_graph(env, st, spmv_blocks(ctx), &loop);
     if (rc != VRG_OK) return rc;
     VRG_CUDA(ctx, cudaGraphLaunch(loop, st));
-    k_digest_partial<<<kDigestBlocks, 256, 0, st>>>(env->d_bake_rgb.as<float>(), 3 * env->luxel_offset.back(), B, n,
-                                                     sc.partials);
-    k_digest_final<<<1, 32, 0, st>>>(sc.partials, kDigestBlocks, sc.digest);
-    VRG_CUDA(ctx, cudaGetLastError());
+    if (digest) {
+        k_digest_partial<<<kDigestBlocks, 256, 0, st>>>(env->d_bake_rgb.as<float>(), 3 * env->luxel_offset.back(), B, n,
+                                                         sc.partials);
+        k_digest_final<<<1, 2 * kDigestBlocks, 0, st>>>(sc.partials, sc.digest);
+        VRG_CUDA(ctx, cudaGetLastError());
+    }
     {
         std::lock_guard<std::mutex> lk(ctx->mu);
-        ctx->launches += 3 + (items > 0 ? 1 : 0);  // plus the loop graph's kernels
+        ctx->launches += 1 + (digest ? 2 : 0) + (items > 0 ? 1 : 0);  // plus the loop graph's kernels
     }
     return VRG_OK;
 }
@@ -842,7 +848,7 @@ int start_slot(vrg_server *s, Slot &sl, Request *r) {
     RelightPlan plan;
     int rc = plan_relight(env, r->edits.data(), (int32_t)r->edits.size(), plan);
     if (rc != VRG_OK) return rc;
-    rc = issue_relight(env, plan, s->max_iters, s->tol, sl.stream, sl.scratch, sl.stage);
+    rc = issue_relight(env, plan, s->max_iters, s->tol, sl.stream, sl.scratch, sl.stage, true);
     if (rc != VRG_OK) return rc;
     env->lights = plan.table;
     char *res = static_cast<char *>(sl.result.ptr);
@@ -921,12 +927,15 @@ int vrg_env_relight(vrg_env *env, const vrg_light_edit *edits, int32_t n, int32_
     if (rc != VRG_OK) return rc;
     RelightState &rs = relight_state(env);
     RelightScratch &sc = rs.sc;
-    rc = issue_relight(env, plan, max_iters, rel_tol, ctx->stream, sc, rs.stage);
+    rc = issue_relight(env, plan, max_iters, rel_tol, ctx->stream, sc, rs.stage, false);
     if (rc != VRG_OK) return rc;
     env->lights = plan.table;
+    // back through the page-locked stage, whose uploads precede it on the stream
     RelightCtl c;
-    VRG_CUDA(ctx, cudaMemcpyAsync(&c, rs.ctl, sizeof c, cudaMemcpyDeviceToHost, ctx->stream));
+    static_assert(sizeof c <= 16 + 24, "fits the smallest request");
+    VRG_CUDA(ctx, cudaMemcpyAsync(rs.stage.ptr, rs.ctl, sizeof c, cudaMemcpyDeviceToHost, ctx->stream));
     VRG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    memcpy(&c, rs.stage.ptr, sizeof c);
     if (out_bounces) *out_bounces = c.iters;
     if (out_delta) *out_delta = c.last_delta;
     env->bake_bounces = c.iters;
