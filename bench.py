@@ -580,17 +580,12 @@ def sub_anyhit(args, lib_ctx, stream, dev, flush, l2, sms):
     dt = time.perf_counter() - t0
     _, rh, rt = s.occlusion_mask(sc.starts, sc.stops, threads=threads, closest=True)
     diff_bits = int(np.unpackbits((got_m ^ rm).view(np.uint8)).sum())
-    tv, tms = lib_ctx.autotune_choice(Context.tune_key("trace_mask", env.num_triangles(), n))
-    hv, hms = lib_ctx.autotune_choice(Context.tune_key("trace_mask_hit", env.num_triangles(), n))
-    # the device's walk, counted by the oracle on the device's tree
-    skip_empty = tv in (12, 13, 14, 15, 16, 17, 18, 19)
+    # a kd walk of the same lines, counted by the oracle on the device's tree
     s.set_tree(*env.walk_tree()[:3])
-    s.set_skip_empty(skip_empty)
     _, st = s.occlusion_mask(sc.starts, sc.stops, threads=threads, stats=True)
     nodes, tris = st[:, 0].mean(), st[:, 1].mean()
     bytes_per_unit = 24 + 1 / 8 + 8 * nodes + 48 * tris
-    prof = "ncu_trace_unit_skip.txt" if tv in (13, 14, 15, 16, 17, 18, 19) else (
-        "ncu_trace_unit_stream.txt" if tv in (6, 7, 9, 10, 11) else "ncu_trace_mask.txt")
+    prof = "ncu_trace_bvh.txt"
     peak, kind = _peaks()
     avg_ms = kms / max(kn, 1)
     env.close()
@@ -601,11 +596,10 @@ def sub_anyhit(args, lib_ctx, stream, dev, flush, l2, sms):
         "config": {"workload": "2^20 shadow lines, both ends uniform in the 4,096-unit room, "
                                "12,300-triangle box room (1,024 boxes), seed 0",
                    "l2": "flushed between steps (512 MiB write)",
-                   "autotune": {"variant": tv, "variant_ms": [round(x, 4) for x in tms]},
                    "setup_acceleration_structure_ms": admit_ms},
         "closest_hit": {"value": round(n / (statistics.mean(hit_ms) * 1e-3) / 1e6, 3),
                         "unit": "Mrays/s", "ms_per_step": round(statistics.mean(hit_ms), 4),
-                        "outputs": "mask + hit index + t", "autotune_variant": hv},
+                        "outputs": "mask + hit index + t"},
         "e2e": {"value": round(n / statistics.median(e2e) / 1e6, 3), "unit": "Mrays/s",
                 "h2d_bytes_per_step": 24 * n, "d2h_bytes_per_step": 4 * ((n + 31) // 32),
                 "statistic": f"median of {len(e2e)} wall-clock steps",
@@ -617,8 +611,8 @@ def sub_anyhit(args, lib_ctx, stream, dev, flush, l2, sms):
                    and bool(np.array_equal(got_t.view(np.uint32), rt.view(np.uint32)))},
         "roofline": _trace_roofline(
             "trace_mask", n, avg_ms, bytes_per_unit, peak, kind, l2, clk, sms, prof,
-            "24 end points + 1/8 mask + 8 per kd node + 48 per triangle test, means of the "
-            "oracle's walk of the device's tree with the device's options", nodes, tris, tv),
+            "24 end points + 1/8 mask + 8 per kd node + 48 per triangle test of the kd walk that the "
+            "four-wide hierarchy replaces, means of the oracle's walk", nodes, tris),
         "cpu_baseline": {"value": round(n / dt / 1e6, 3), "unit": "Mrays/s", "cores": threads,
                          "kind": "port", "sample": f"all {n} lines, the reference's SAH tree"},
         "clocks": clk,

@@ -15,7 +15,8 @@
  * pointers.  The trace entry points (vrg_env_occlusion_mask,
  * vrg_env_trace_closest, vrg_env_test_line_does_hit_sky) read page-locked
  * host inputs (cudaHostAlloc / cudaHostRegister) in place over the CPU-GPU
- * link; other host buffers are copied in and out inside the call.
+ * link; other host buffers are copied in and out inside the call, those of a
+ * small call (up to 1 MiB together) through page-locked memory of the context.
  *
  * Threading: a context may be shared by several host threads; each
  * environment serialises its own calls with a mutex.
@@ -127,8 +128,7 @@ int vrg_ctx_reset_stats(vrg_ctx *ctx);
 int64_t vrg_ctx_launch_count(const vrg_ctx *ctx);
 
 /* Per-scene-size autotuning (no reference counterpart).  Tuned launch
- * sites ("trace_mask", "trace_mask_hit", "direct_luxels", "transfer_rows",
- * "bounce_spmv", "batch_gather") offer variants that give identical results (the bounce
+ * sites ("direct_luxels", "transfer_rows", "bounce_spmv", "batch_gather") offer variants that give identical results (the bounce
  * variants: the same sums); the first launch in a bucket
  * "<site>/t<log2 triangles>/n<log2 work items>" times each twice on the real
  * input and keeps the fastest.  On by default; off, or inside a stream
@@ -442,11 +442,11 @@ int vrg_env_make_transfers(vrg_env *env, const float *dirs_local, int32_t k, int
 /* CSR copy-out: row_ptr[leaves+1], col[nnz], weight[nnz] (= hits / k). */
 int vrg_env_get_transfers(const vrg_env *env, int64_t *row_ptr, int32_t *col, float *weight);
 /* The last build's ray count k, entry count, and how many of its rows had
- * more distinct targets than the shared-memory row table holds (those rows
+ * more distinct targets than the first pass stages per row (those rows
  * are rebuilt by a global-memory sort; the CSR is the same either way).
  * (no reference counterpart: transfer building is absent there) */
 int vrg_env_transfer_info(const vrg_env *env, int32_t *k, int64_t *nnz, int64_t *overflow_rows);
-/* Distinct targets a transfer row may collect in its shared-memory table
+/* Distinct targets a transfer row may stage on the first pass
  * before the row is rebuilt by the global-memory sort (default and maximum
  * 7168; a lower limit sends more rows down that path, which tests use).
  * (no reference counterpart) */

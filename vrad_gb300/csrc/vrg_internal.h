@@ -95,7 +95,7 @@ struct vrg_ctx {
     int64_t launches = 0;
     bool autotune = true;
     uint64_t hbm_reserve = (uint64_t)1 << 30;  // kept free when admitting a relight scene
-    int32_t xfer_table_limit = 7168;            // distinct targets per transfer row held in shared memory
+    int32_t xfer_table_limit = 7168;            // distinct targets of a transfer row staged on the first pass
     // kStageBytes of page-locked memory that kernels read and write in place
     // (null: not to be had), one call at a time
     std::mutex stage_mu;
