@@ -294,10 +294,10 @@ def _event_ms(stream, fn, steps, flush):
 
 def _trace_roofline(kernel, units, avg_ms, bytes_per_unit, hbm_peak, hbm_kind, l2, clk, sms,
                     prof, bytes_model, nodes, tris, variant=None):
-    """Roofline record of a traversal kernel.  Its algorithmic bytes (kd
-    nodes and leaf records) are served from L1 and L2, so the governing roof
-    is instruction issue; the L2 and HBM fractions are given beside it, HBM
-    from the DRAM bytes ncu counted for the same kernel.  The instruction
+    """Roofline record of a traversal kernel: the governing roof is
+    instruction issue.  Beside it the bytes that a kd walk of the same lines
+    would read (nodes and leaf records) against the L2 rate, and HBM from the
+    DRAM bytes ncu counted for the same kernel.  The instruction
     count is the tuned variant's own (`warp_instructions_per_unit_v<n>`)
     where the summary has it."""
     alg = bytes_per_unit * units / (avg_ms * 1e-3) / 1e9
@@ -315,7 +315,9 @@ def _trace_roofline(kernel, units, avg_ms, bytes_per_unit, hbm_peak, hbm_kind, l
     rec = {"bound": "issue", "kernel": kernel, "kernel_ms": round(avg_ms, 4),
            "bytes_per_unit": round(bytes_per_unit, 2), "bytes_model": bytes_model,
            "nodes_per_unit": round(float(nodes), 3), "tris_per_unit": round(float(tris), 3),
-           "l2": {"achieved": round(alg, 1), "peak": round(l2, 1) if l2 else None, "unit": "GB/s",
+           # bytes of the kd walk that the maps and the hierarchy replace, per second:
+           # above the L2 rate where the kernel reads fewer
+           "walk_l2": {"achieved": round(alg, 1), "peak": round(l2, 1) if l2 else None, "unit": "GB/s",
                   "frac": round(alg / l2, 4) if l2 else None,
                   "peak_source": "L2-resident read kernel (probe.cu), timed in this run"},
            "hbm": {"achieved": round(traffic / (avg_ms * 1e-3) / 1e9, 1) if traffic else None,
@@ -327,8 +329,8 @@ def _trace_roofline(kernel, units, avg_ms, bytes_per_unit, hbm_peak, hbm_kind, l
         rec.update({"achieved": issue["achieved"], "peak": issue["peak"], "unit": issue["unit"],
                     "frac": issue["frac"], "issue": issue})
     else:
-        rec.update({"achieved": rec["l2"]["achieved"], "peak": rec["l2"]["peak"], "unit": "GB/s",
-                    "frac": rec["l2"]["frac"], "bound": "l2"})
+        rec.update({"achieved": rec["walk_l2"]["achieved"], "peak": rec["walk_l2"]["peak"], "unit": "GB/s",
+                    "frac": rec["walk_l2"]["frac"], "bound": "l2"})
     return rec
 
 
