@@ -566,7 +566,7 @@ bool use_sky_map(vrg_env *env, int64_t points, bool repaid) {
     // build 4.4 / 4.6 / 5.8 ms.  At least 96 cells an axis: where boxes are few
     // most lines pass them, and it is the wide cells around a sample's own box
     // that leave them undecided.  A gather of a 2,064-triangle brush map takes
-    // 0.49 / 0.41 / 0.37 ms with 80 / 96 / 128 cells (first 1.43 / 1.40 / 1.65),
+    // 0.49 / 0.41 / 0.37 ms with 72 / 96 / 128 cells (first 1.43 / 1.40 / 1.65),
     // twelve scenes of 64 to 4,096 faces 4.0 / 3.8 / 3.55 ms at least 32 / 96 / 128
     // (first 14.0 / 14.5 / 16.1).
     const int n = std::min(512, std::max(96, (int)std::sqrt(3.0 * (double)nt) & ~7));

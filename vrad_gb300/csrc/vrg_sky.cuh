@@ -133,7 +133,7 @@ __device__ __forceinline__ float sky_sweep(const DevScene &s, const SkyView &sv,
 // normal faces are listed once for all lanes with their cosines, for the two
 // normals of a warp at the end of a face at a time.  The room's sky takes
 // 1.66 ms (2.24 with every lane asking all 162 for their cosine, 15.4 by the
-// walk), with 157 x 157 cells per direction.  Queueing the undecided lines for
+// walk), with 152 x 152 cells per direction.  Queueing the undecided lines for
 // a full warp at a time cost more in locality than it saved: 1.79 ms, and a
 // batch of 48-unit scenes 3.0 instead of 2.7.
 __device__ __forceinline__ float sky_fraction(const DevScene &s, const SkyView &sv, unsigned lanes, float px, float py,
