@@ -322,7 +322,9 @@ struct Builder {
         }
         const uint32_t at = (uint32_t)out.size();
         out.emplace_back();
-        deepest = std::max(deepest, stack + n);
+        // three siblings wait while a walk follows one child, whatever n is: a
+        // ray whose reciprocal is no number passes the unused boxes too
+        deepest = std::max(deepest, stack + 4);
         uint32_t word[4];
         for (int c = 0; c < 4; c++) {
             word[c] = kBvhLeafBit;

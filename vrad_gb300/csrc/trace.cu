@@ -91,15 +91,15 @@ __global__ void __launch_bounds__(kThreads, MINB) k_bvh(DevScene s, BvhView bv, 
                         load3(q.b, ri, ray.dx, ray.dy, ray.dz);
                         t0 = __ldg(q.tmin + ri);
                         len = __ldg(q.tmax + ri);
-                        rp = box_ray(ray, ray_slack(s.g, ray.ox, ray.oy, ray.oz));
-                        active = bv.nodes && t0 <= len;
+                        rp = box_ray(s.g, ray, ray_slack(s.g, ray.ox, ray.oy, ray.oz));
+                        active = bv.nodes && t0 <= len && has_direction(ray);
                     } else {
                         float sx, sy, sz, ex, ey, ez;
                         load3(q.a, ri, sx, sy, sz);
                         load3(q.b, ri, ex, ey, ez);
                         const LinePlan p = plan_line(s, make_line(sx, sy, sz, ex, ey, ez));
                         ray = p.ray;
-                        rp = box_ray(ray, p.slack);
+                        rp = box_ray(s.g, ray, p.slack);
                         len = p.len;
                         any_limit = p.any_limit;
                         active = bv.nodes && !p.trivial;

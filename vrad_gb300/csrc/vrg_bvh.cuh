@@ -16,26 +16,50 @@
 
 namespace vrg {
 
+__device__ __forceinline__ float box_rcp(float d) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+    return r;
+}
+
 // A ray against boxes: per axis the reciprocal direction and the origin's
 // distance to a plane that the ray enters or leaves by, moved by the slab.
+//
+// bvh_step multiplies the reciprocal by up to 2^23 steps of a node, a 60th of
+// the scene's scale at most, and that has to stay finite: an infinity of the
+// wrong sign closes every box.  So no component counts as less than 2^-28 of
+// the largest.  A hit inside the scene is at most scale + |origin| away along
+// the largest axis, so this moves it sideways by less than a thousandth of the
+// slab.  A direction too short or too long for the rest (the product is then
+// 2^120 at most) gets no number for its reciprocal: it passes every box, and the
+// exact tests decide alone.
 struct BoxRay {
     float inv[3], in[3], out[3];
     uint32_t neg;  // bit a: the direction's a component is negative
 };
-__device__ __forceinline__ BoxRay box_ray(const Ray &ray, float slack) {
+__device__ __forceinline__ BoxRay box_ray(const SceneGeom &g, const Ray &ray, float slack) {
     BoxRay r;
     const float o[3] = {ray.ox, ray.oy, ray.oz}, d[3] = {ray.dx, ray.dy, ray.dz};
+    const float most = fmaxf(fabsf(d[0]), fmaxf(fabsf(d[1]), fabsf(d[2])));
+    const bool fits = most >= fmaxf(g.scale * 0x1p-75f, 0x1p-90f) && most <= 0x1p60f;
+    const float least = most * 0x1p-28f;
     r.neg = 0u;
 #pragma unroll
     for (int a = 0; a < 3; a++) {
         const bool neg = signbit(d[a]);
         r.neg |= (neg ? 1u : 0u) << a;
-        r.inv[a] = trav_rcp(d[a]);
+        r.inv[a] = fits ? box_rcp(fabsf(d[a]) < least ? copysignf(least, d[a]) : d[a]) : __int_as_float(0x7fc00000);
         const float sd = neg ? -slack : slack;
         r.in[a] = -sd - o[a];
         r.out[a] = sd - o[a];
     }
     return r;
+}
+
+// A direction of no length meets no triangle: the quotient that the exact test
+// takes is infinite or no number.
+__device__ __forceinline__ bool has_direction(const Ray &ray) {
+    return ray.dx != 0.0f || ray.dy != 0.0f || ray.dz != 0.0f;
 }
 
 // 2^23 + byte c of w, as a float.
@@ -133,8 +157,8 @@ __device__ __forceinline__ int32_t bvh_trace(const DevScene &s, const BvhView &b
     int32_t best = -1;
     float best_t = kInf;
     uint2 stk[kBvhStack];
-    if (bv.nodes && tmin <= tmax) {
-        const BoxRay rp = box_ray(ray, slack);
+    if (bv.nodes && tmin <= tmax && has_direction(ray)) {
+        const BoxRay rp = box_ray(s.g, ray, slack);
         uint32_t cur = 0u;
         int sp = 0;
         for (;;) {
