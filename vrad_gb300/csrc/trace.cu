@@ -188,6 +188,8 @@ __global__ void __launch_bounds__(32 * kFewWarps) k_few(DevScene s, QueryArgs q,
     const int share = (ntris + slices - 1) / slices;
     const int first = blockIdx.y * share + wid, end = min(ntris, ((int)blockIdx.y + 1) * share);
     const float4 *planes = s.leaf_planes + base, *edges = s.leaf_edges + 2 * base;
+    // whether a quotient's sign alone puts it out of range
+    const bool ahead = t0 >= 0.0f && (Q != kQClosest || fabsf(ray.dx) + fabsf(ray.dy) + fabsf(ray.dz) <= 1e38f);
     int32_t best = -1;
     float best_t = t1;  // the first hit must be below
     for (int k0 = first; k0 < end; k0 += kFewWarps * kFewUnroll) {
@@ -205,7 +207,7 @@ __global__ void __launch_bounds__(32 * kFewWarps) k_few(DevScene s, QueryArgs q,
             // t < 0 where that is out of range, or past the best hit by more
             // than the quotient's rounding
             const bool neg = ((__float_as_uint(num) ^ __float_as_uint(den)) >> 31) != 0u;
-            if (neg ? t0 >= 0.0f && fabsf(num) > 1e-30f : fabsf(num) > best_t * fabsf(den) * 1.000001f) continue;
+            if (neg ? ahead && fabsf(num) > kSureNumerator : fabsf(num) > best_t * fabsf(den) * 1.000001f) continue;
             const float t = rdiv(num, den);
             if (!(t >= t0 && t < t1 && t <= best_t)) continue;
             const float4 w2 = __ldg(edges + 2 * (size_t)k + 1);

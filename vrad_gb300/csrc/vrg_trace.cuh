@@ -246,6 +246,10 @@ __device__ __forceinline__ float4 leaf_load(const float4 *p) {
     return v;
 }
 
+// No finite divisor makes a numerator above this round to -0, which a start of
+// 0 accepts.
+constexpr float kSureNumerator = 1e-6f;
+
 template <int MODE, int OPT = 0>
 __device__ __forceinline__ bool tri_test(const DevScene &s, const Ray &ray, float tmin, float tmax,
                                          int32_t skip, float any_limit, const float4 w0, size_t k,
@@ -254,8 +258,8 @@ __device__ __forceinline__ bool tri_test(const DevScene &s, const Ray &ray, floa
     const float on = dot3r(w0.x, w0.y, w0.z, ray.ox, ray.oy, ray.oz);
     const float num = rsub(w0.w, on);
     if (OPT & kOptSign) {
-        // signs differ: t < 0 (above 1e-30 the quotient does not round to -0)
-        if (((__float_as_uint(num) ^ __float_as_uint(den)) >> 31) && fabsf(num) > 1e-30f) return false;
+        // signs differ: t < 0
+        if (((__float_as_uint(num) ^ __float_as_uint(den)) >> 31) && fabsf(num) > kSureNumerator) return false;
     }
     const float t = rdiv(num, den);
     if (!(t >= tmin && t < tmax)) return false;
