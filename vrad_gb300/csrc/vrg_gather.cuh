@@ -27,7 +27,8 @@ __device__ __forceinline__ uint64_t splitmix(uint64_t seed, uint64_t i) {
     return z ^ (z >> 31);
 }
 
-// The box around a warp's sample points, and whether they share their normal.
+// The box around a warp's sample points, and whether they share their normal
+// (and are numbers, so that the box holds them all).
 struct PointBox {
     float lo[3], hi[3];
     bool one;
@@ -52,7 +53,9 @@ __device__ __forceinline__ PointBox point_box(unsigned lanes, float px, float py
     }
     const int lead = __ffs(lanes) - 1;
     const float lx = __shfl_sync(lanes, nx, lead), ly = __shfl_sync(lanes, ny, lead), lz = __shfl_sync(lanes, nz, lead);
-    b.one = __all_sync(lanes, nx == lx && ny == ly && nz == lz);
+    // (a coordinate that is no number takes a bound's place and hides the others')
+    b.one = __all_sync(lanes, nx == lx && ny == ly && nz == lz) && b.lo[0] <= b.hi[0] && b.lo[1] <= b.hi[1] &&
+            b.lo[2] <= b.hi[2];
     return b;
 }
 
