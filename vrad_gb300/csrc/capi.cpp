@@ -754,6 +754,7 @@ int vrg_env_set_faces(vrg_env *env, int32_t nfaces, const float *corner, const f
     for (int64_t i = 0; i < 3 * (int64_t)nfaces; i++)
         for (const float c : {corner[i], corner[i] + u[i], corner[i] + v[i], corner[i] + u[i] + v[i]})
             env->faces_inside = env->faces_inside && std::fabs(c) <= reach && std::fabs(normal[i]) <= 2.0f;
+    env->faces_in_sky_range = faces_in_sky_range(env);
     TRY(upload(ctx, env->d_faces, recs.data(), recs.size() * sizeof(FaceRec)));
     TRY(upload(ctx, env->d_luxel_offset, env->luxel_offset.data(), env->luxel_offset.size() * 8));
     TRY(upload(ctx, env->d_tri_face, env->tri_face.data(), std::max<size_t>(1, env->tri_face.size()) * 4));

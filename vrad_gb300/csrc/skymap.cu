@@ -356,13 +356,16 @@ __global__ void __launch_bounds__(kThreads) k_sky_sort(const uint2 *__restrict__
     }
 }
 
+// How far the maps reach past the scene's bounds: eight times the walk's slab
+// half-thickness for a point as far out as three times the scene's largest
+// coordinate.
+double sky_margin(const SceneGeom &g) { return 8.0 * std::ldexp(1.0, -17) * (3.0 * (double)g.scale + 1.0); }
+
 // The directions' maps over the scene's bounds, n cells per axis.
 void make_dirs(const vrg_env *env, int n, std::vector<SkyDir> &out) {
     static const float anorms[kNumAnorms * 3] = VRG_ANORMS_INIT;
     const SceneGeom &g = env->geom;
-    // eight times the walk's slab half-thickness for a point as far out as
-    // three times the scene's largest coordinate
-    const double m = 8.0 * std::ldexp(1.0, -17) * (3.0 * (double)g.scale + 1.0);
+    const double m = sky_margin(g);
     out.resize(kNumAnorms);
     for (int j = 0; j < kNumAnorms; j++) {
         SkyDir &o = out[j];
@@ -544,13 +547,27 @@ SkyView sky_view(const vrg_env *env) {
     return v;
 }
 
+bool faces_in_sky_range(const vrg_env *env) {
+    const SceneGeom &g = env->geom;
+    const double m = sky_margin(g);
+    for (int c = 0; c < 3; c++) {
+        const double far = 128.0 * ((double)g.bmax[c] - g.bmin[c] + 2.0 * m) - 1.0;
+        for (int32_t f = 0; f < env->nfaces; f++) {
+            const double p = env->f_corner[3 * f + c], u = env->f_u[3 * f + c], v = env->f_v[3 * f + c];
+            const double lo = p + std::min(0.0, u) + std::min(0.0, v), hi = p + std::max(0.0, u) + std::max(0.0, v);
+            if (!(lo >= g.bmin[c] - far && hi <= g.bmax[c] + far)) return false;
+        }
+    }
+    return true;
+}
+
 int64_t sky_map_points(const vrg_env *env) { return std::max<int64_t>(24 * env->geom.ntris, 40000); }
 
 bool use_sky_map(vrg_env *env, int64_t points, bool repaid) {
     vrg_ctx *ctx = env->ctx;
     bool ambient = false;
     for (const vrg_light &l : env->lights) ambient = ambient || l.type == VRG_EMIT_SKYAMBIENT;
-    if (!ambient || env->sky_n < 0 || !env->faces_inside) return false;
+    if (!ambient || env->sky_n < 0 || !env->faces_inside || !env->faces_in_sky_range) return false;
     if (env->sky_n > 0) return true;
     const int64_t nt = env->geom.ntris;
     // a build costs about what 24 sample points per triangle cost to walk, and

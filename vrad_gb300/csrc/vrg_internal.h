@@ -196,6 +196,7 @@ struct vrg_env {
     std::vector<int32_t> f_nu, f_nv, tri_face;
     std::vector<int64_t> luxel_offset;
     bool faces_inside = false;  // every face lies within the scene's coordinates
+    bool faces_in_sky_range = false;  // and within the depths that the sky maps' lookup can tell apart
     vrg::DevBuf d_faces, d_luxel_offset, d_tri_face;
 
     // patches / transfers / bounce
@@ -296,6 +297,9 @@ int launch_test_lines(vrg_env *env, const float *start, const float *stop, int64
 // scene's faces go through the maps (built here when the points repay it), and
 // the maps as the kernels read them.
 bool use_sky_map(vrg_env *env, int64_t points, bool repaid = false);
+// The lookup rounds a depth by adding 1.5 * 2^23 to it, which keeps the order
+// down to -2^23 levels, 129 times the map's 65,000; farther out it wraps.
+bool faces_in_sky_range(const vrg_env *env);
 int64_t sky_map_points(const vrg_env *env);  // sample points that repay building the maps
 SkyView sky_view(const vrg_env *env);
 // Luxel samples of every face, then (optionally) npts extra sample points

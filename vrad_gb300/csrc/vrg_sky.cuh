@@ -17,7 +17,9 @@ static __constant__ float c_anorms[kNumAnorms * 3] = VRG_ANORMS_INIT;
 // Cell and depth of a point in direction j's map; false outside the map,
 // where no triangle is.  Coordinates round to integers by adding 1.5 * 2^23
 // (the cell coordinates are stored half a cell low, so that rounding to the
-// nearest finds the cell): the margins of the bounds cover both roundings.
+// nearest finds the cell): the margins of the bounds cover both roundings.  A
+// value below -2^23 would wrap: such a cell is outside the map all the same, and
+// no sample point lies at such a depth (faces_in_sky_range).
 __device__ __forceinline__ int round_bits(float v) {
     return (int)(__float_as_uint(v + 12582912.0f) - 0x4b400000u);
 }
