@@ -273,8 +273,10 @@ __global__ void __launch_bounds__(kThreads) k_sky_large(const SkyTri *__restrict
 
 // Between counting and filling: each cell takes its run of the pool (block
 // scan, one atomic per block), the two bounds are packed, and `clear` becomes
-// the fill counter.
-__global__ void __launch_bounds__(256) k_sky_pack(SkyGrids g, int64_t cells, unsigned int *__restrict__ cursor) {
+// the fill counter.  The cursor counts in 64 bits: coincident triangles put
+// thousands of entries into every cell, and past 2^32 the runs' starts would
+// wrap (build gives up on such maps before anything is filled).
+__global__ void __launch_bounds__(256) k_sky_pack(SkyGrids g, int64_t cells, unsigned long long *__restrict__ cursor) {
     __shared__ uint32_t warp_sum[8];
     __shared__ uint32_t base_sh;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -296,7 +298,7 @@ __global__ void __launch_bounds__(256) k_sky_pack(SkyGrids g, int64_t cells, uns
                 warp_sum[k] = sum;
                 sum += v;
             }
-            base_sh = sum ? atomicAdd(cursor, sum) : 0u;
+            base_sh = sum ? (uint32_t)atomicAdd(cursor, (unsigned long long)sum) : 0u;
         }
         __syncthreads();
         if (c < cells) {
@@ -467,7 +469,7 @@ int build(vrg_env *env, int n) {
     SkyGrids g{};
     g.info = reinterpret_cast<uint2 *>(base + vbytes);
     g.bound = reinterpret_cast<uint32_t *>(base + vbytes + 8 * cells);
-    unsigned int *cursor = tmp.as<unsigned int>();
+    unsigned long long *cursor = tmp.as<unsigned long long>();
     g.clear = tmp.as<uint32_t>() + 64;
     uint32_t *large = g.clear + cells * (has_sky ? 4 : 1);
     if (has_sky) {
@@ -486,7 +488,7 @@ int build(vrg_env *env, int n) {
     unsigned int passes = 0;  // each pass counts its large splats in a word of its own after the cursor
     auto cells_pass = [&](auto kernel, auto kernel_large, int64_t first, int64_t count) {
         const SkyTri *t = d_tris + first;
-        unsigned int *nlarge = cursor + ++passes;
+        unsigned int *nlarge = reinterpret_cast<unsigned int *>(cursor + 1) + passes++;
         // a small scene's pairs go to more warps, fewer each
         const int64_t warps = (int64_t)ctx->num_sms * 48;
         const int batch = (int)std::min<int64_t>(32, std::max<int64_t>(1, count * kNumAnorms / warps));
@@ -513,9 +515,10 @@ int build(vrg_env *env, int n) {
         g, (int64_t)cells, cursor);
     VRG_CUDA(ctx, cudaGetLastError());
     timing_end(ctx, "sky_map", ev);
-    unsigned int entries = 0;
-    VRG_CUDA(ctx, cudaMemcpyAsync(&entries, cursor, 4, cudaMemcpyDeviceToHost, st));
+    uint64_t entries = 0;
+    VRG_CUDA(ctx, cudaMemcpyAsync(&entries, cursor, 8, cudaMemcpyDeviceToHost, st));
     VRG_CUDA(ctx, cudaStreamSynchronize(st));
+    if (!sky_pool_indexable(entries)) return fail(ctx, VRG_ERR_UNSUPPORTED, "sky maps of more than 2^32 entries");
     VRG_CUDA(ctx, env->d_sky_pool.reserve(8 * (size_t)entries));
     g.pool = env->d_sky_pool.as<uint2>();
     VRG_CUDA(ctx, cells_pass(k_sky_cells<kFill>, k_sky_large<kFill>, 0, nt));

@@ -300,6 +300,8 @@ bool use_sky_map(vrg_env *env, int64_t points, bool repaid = false);
 // The lookup rounds a depth by adding 1.5 * 2^23 to it, which keeps the order
 // down to -2^23 levels, 129 times the map's 65,000; farther out it wraps.
 bool faces_in_sky_range(const vrg_env *env);
+// Cells hold their run's first pool entry and an end in 32 bits.
+inline bool sky_pool_indexable(uint64_t entries) { return entries <= 0xffffffffull; }
 int64_t sky_map_points(const vrg_env *env);  // sample points that repay building the maps
 SkyView sky_view(const vrg_env *env);
 // Luxel samples of every face, then (optionally) npts extra sample points
