@@ -416,14 +416,35 @@ void make_dirs(const vrg_env *env, int n, std::vector<SkyDir> &out) {
     }
 }
 
+static_assert(sizeof(SkyTri) == kSkyTriBytes && sizeof(SkyDir) == kSkyDirBytes, "SkyMapSizes counts them");
+
+// Whether `bytes` more leave the context's reserve free.
+bool leaves_reserve(vrg_ctx *ctx, size_t bytes) {
+    size_t free_b = 0, total_b = 0;
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return false;
+    }
+    std::lock_guard<std::mutex> lk(ctx->mu);
+    return free_b >= bytes && free_b - bytes >= ctx->hbm_reserve;
+}
+
 // Builds env's maps with the context's scratch, which one build at a time
 // holds until its kernels are done.
 int build(vrg_env *env, int n) {
     vrg_ctx *ctx = env->ctx;
     std::lock_guard<std::mutex> scratch(ctx->scratch_mu);
+    DevBuf &tmp = ctx->scratch;
+    struct Trim {  // however the build ends
+        DevBuf &buf;
+        ~Trim() {
+            if (buf.bytes > kScratchKept) buf.release();
+        }
+    } trim{tmp};
     cudaStream_t st = ctx->stream;
     const int64_t nt = env->geom.ntris;
-    const size_t cells = (size_t)kNumAnorms * n * n;
+    const SkyMapSizes sizes(nt, n, env->geom.has_sky != 0);
+    const size_t cells = sizes.cells;
     // any leaf entry of a triangle holds its record; ids of -1 are the lines'
     // skip id, which no line hits
     const std::vector<int32_t> &refs = env->walk_tree.refs;
@@ -454,17 +475,12 @@ int build(vrg_env *env, int n) {
         view[4 * j + 2] = dirs[j].gd;
         view[4 * j + 3] = make_float4(dirs[j].d[0], dirs[j].d[1], dirs[j].d[2], 0.0f);
     }
-    const bool has_sky = nsky > 0;
-    const int64_t pairs = nt * kNumAnorms;
-    const size_t vbytes = view.size() * sizeof(float4);
-    VRG_CUDA(ctx, env->d_sky_cells.reserve(vbytes + 12 * cells));
-    // scratch [counters | grids | large pairs | triangles | directions]
-    const size_t tri_at = (256 + 4 * cells * (has_sky ? 4 : 1) + 4 * (size_t)pairs + 15) & ~(size_t)15;
-    const size_t dir_at = tri_at + sizeof(SkyTri) * (size_t)nt;
-    DevBuf &tmp = ctx->scratch;
-    VRG_CUDA(ctx, tmp.reserve(dir_at + sizeof(SkyDir) * kNumAnorms));
-    SkyTri *d_tris = reinterpret_cast<SkyTri *>(tmp.as<char>() + tri_at);
-    SkyDir *d_dirs = reinterpret_cast<SkyDir *>(tmp.as<char>() + dir_at);
+    const bool has_sky = env->geom.has_sky != 0;
+    const size_t vbytes = sizes.view;
+    VRG_CUDA(ctx, env->d_sky_cells.reserve(sizes.kept));
+    VRG_CUDA(ctx, tmp.reserve(sizes.scratch));
+    SkyTri *d_tris = reinterpret_cast<SkyTri *>(tmp.as<char>() + sizes.tri_at);
+    SkyDir *d_dirs = reinterpret_cast<SkyDir *>(tmp.as<char>() + sizes.dir_at);
     char *base = env->d_sky_cells.as<char>();
     SkyGrids g{};
     g.info = reinterpret_cast<uint2 *>(base + vbytes);
@@ -519,6 +535,7 @@ int build(vrg_env *env, int n) {
     VRG_CUDA(ctx, cudaMemcpyAsync(&entries, cursor, 8, cudaMemcpyDeviceToHost, st));
     VRG_CUDA(ctx, cudaStreamSynchronize(st));
     if (!sky_pool_indexable(entries)) return fail(ctx, VRG_ERR_UNSUPPORTED, "sky maps of more than 2^32 entries");
+    if (!leaves_reserve(ctx, 8 * (size_t)entries)) return fail(ctx, VRG_ERR_NOMEM, "no room for the sky maps' lists");
     VRG_CUDA(ctx, env->d_sky_pool.reserve(8 * (size_t)entries));
     g.pool = env->d_sky_pool.as<uint2>();
     VRG_CUDA(ctx, cells_pass(k_sky_cells<kFill>, k_sky_large<kFill>, 0, nt));
@@ -529,7 +546,6 @@ int build(vrg_env *env, int n) {
     timing_end(ctx, "sky_map", ev);
     // later calls may launch on another stream, and the scratch is free again
     VRG_CUDA(ctx, cudaStreamSynchronize(st));
-    if (tmp.bytes > kScratchKept) tmp.release();
     env->sky_n = n;
     return VRG_OK;
 }
@@ -590,19 +606,10 @@ bool use_sky_map(vrg_env *env, int64_t points, bool repaid) {
     // twelve scenes of 64 to 4,096 faces 4.0 / 3.8 / 3.55 ms at least 32 / 96 / 128
     // (first 14.0 / 14.5 / 16.1).
     const int n = std::min(512, std::max(96, (int)std::sqrt(3.0 * (double)nt) & ~7));
-    // the map and its scratch, with room for the lists, inside what the
-    // context may take
-    const size_t need = (size_t)kNumAnorms * n * n * 40 + (size_t)nt * 64;
-    size_t free_b = 0, total_b = 0;
-    uint64_t reserve;
-    {
-        std::lock_guard<std::mutex> lk(ctx->mu);
-        reserve = ctx->hbm_reserve;
-    }
-    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || free_b < need || free_b - need < reserve) {
-        (void)cudaGetLastError();
-        return false;
-    }
+    // the maps and their scratch inside what the context may take; the lists,
+    // whose size the build finds out, are asked for there
+    const SkyMapSizes sizes(nt, n, env->geom.has_sky != 0);
+    if (!leaves_reserve(ctx, sizes.kept + sizes.scratch)) return false;
     std::string said;
     {
         std::lock_guard<std::mutex> lk(ctx->mu);

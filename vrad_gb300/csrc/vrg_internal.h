@@ -302,6 +302,21 @@ bool use_sky_map(vrg_env *env, int64_t points, bool repaid = false);
 bool faces_in_sky_range(const vrg_env *env);
 // Cells hold their run's first pool entry and an end in 32 bits.
 inline bool sky_pool_indexable(uint64_t entries) { return entries <= 0xffffffffull; }
+// Bytes of maps of n x n cells over nt triangles, apart from their pool: what
+// stays with the scene [directions | cells], and what the build takes of the
+// context's scratch [counters | grids | large pairs | triangles | directions].
+constexpr size_t kSkyTriBytes = 48, kSkyDirBytes = 112;
+struct SkyMapSizes {
+    size_t cells, view, kept, tri_at, dir_at, scratch;
+    SkyMapSizes(int64_t nt, int n, bool has_sky) {
+        cells = (size_t)kNumAnorms * n * n;
+        view = 4 * kNumAnorms * 16;
+        kept = view + 12 * cells;
+        tri_at = (256 + 4 * cells * (has_sky ? 4 : 1) + 4 * kNumAnorms * (size_t)nt + 15) & ~(size_t)15;
+        dir_at = tri_at + kSkyTriBytes * (size_t)nt;
+        scratch = dir_at + kSkyDirBytes * kNumAnorms;
+    }
+};
 int64_t sky_map_points(const vrg_env *env);  // sample points that repay building the maps
 SkyView sky_view(const vrg_env *env);
 // Luxel samples of every face, then (optionally) npts extra sample points
