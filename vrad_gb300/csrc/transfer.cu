@@ -934,7 +934,10 @@ int prepare_tiles(vrg_env *env, const std::vector<float> &dirs, int32_t k, TileS
             spheres[c] = ball(vs);
         }
         const size_t sbytes = 16 * (nc + n);
-        VRG_CUDA(ctx, env->d_tile_scene.reserve(sbytes + sizeof(TileTri) * tris.size()));
+        if (env->d_tile_scene.reserve(sbytes + sizeof(TileTri) * tris.size()) != cudaSuccess) {
+            (void)cudaGetLastError();
+            return VRG_OK;  // no room: the rows are walked
+        }
         VRG_CUDA(ctx, cudaMemcpyAsync(env->d_tile_scene.ptr, spheres.data(), sbytes, cudaMemcpyHostToDevice, st));
         VRG_CUDA(ctx, cudaMemcpyAsync(env->d_tile_scene.as<char>() + sbytes, tris.data(), sizeof(TileTri) * tris.size(),
                                       cudaMemcpyHostToDevice, st));
@@ -1041,25 +1044,46 @@ int run_make_transfers(vrg_env *env, const float *dirs_local, int32_t k) {
     // rows go through in chunks whose staging stays near 1 GiB
     const int64_t chunk =
         std::max<int64_t>(1, std::min<int64_t>(rows, ((int64_t)1 << 30) / (8 * (int64_t)tsize)));
-    // blocks that count at once: what the SMs hold of 256 threads, fewer where
-    // the leaves are so many that their counters would pass 8 GiB
-    const int64_t grid_max =
-        std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(rows, (int64_t)ctx->num_sms * 8),
-                                               ((int64_t)8 << 30) / (4 * scratch_stride)));
-    // the context's scratch [staged columns | counts | counters | row sizes |
-    // directions | cones | spreads]; this call waits for its kernels
+    // the context's scratch [staged columns | counts | row sizes | directions |
+    // cones | spreads | counters]; this call waits for its kernels
     std::lock_guard<std::mutex> scratch(ctx->scratch_mu);
+    struct Trim {  // however the call ends
+        DevBuf &buf;
+        ~Trim() {
+            if (buf.bytes > kScratchKept) buf.release();
+        }
+    } trim{ctx->scratch};
     size_t at = 0;
     auto part = [&at](size_t bytes) {
         const size_t here = at;
         at = (at + bytes + 255) & ~(size_t)255;
         return here;
     };
-    const size_t stage = 4 * (size_t)chunk * tsize, count_bytes = 4 * (size_t)(grid_max * scratch_stride);
-    const size_t at_col = part(stage), at_cnt = part(stage), at_counters = part(count_bytes),
-                 at_nnz = part(4 * (size_t)chunk), at_dirs = part(12 * (size_t)k), at_cones = part(16 * cones.size()),
-                 at_spread = part(8 * spread.size());
-    VRG_CUDA(ctx, ctx->scratch.reserve(at));
+    const size_t stage = 4 * (size_t)chunk * tsize;
+    const size_t at_col = part(stage), at_cnt = part(stage), at_nnz = part(4 * (size_t)chunk),
+                 at_dirs = part(12 * (size_t)k), at_cones = part(16 * cones.size()), at_spread = part(8 * spread.size()),
+                 at_counters = at;
+    const size_t row_counters = 4 * (size_t)scratch_stride;  // of one block
+    int64_t grid_max = transfer_blocks(rows, ctx->num_sms, row_counters, (uint64_t)8 << 30, 0);
+    if (at_counters + grid_max * row_counters > ctx->scratch.bytes) {
+        // a larger scratch than the context holds: fewer blocks where memory is short
+        size_t free_b = 0, total_b = 0;
+        VRG_CUDA(ctx, cudaMemGetInfo(&free_b, &total_b));
+        uint64_t reserve;
+        {
+            std::lock_guard<std::mutex> lk(ctx->mu);
+            reserve = ctx->hbm_reserve;
+        }
+        free_b += ctx->scratch.bytes;
+        grid_max = transfer_blocks(rows, ctx->num_sms, row_counters, free_b > at_counters ? free_b - at_counters : 0, reserve);
+        for (;; grid_max = (grid_max + 1) / 2) {
+            const cudaError_t e = ctx->scratch.reserve(at_counters + grid_max * row_counters);
+            if (e == cudaSuccess) break;
+            (void)cudaGetLastError();
+            if (e != cudaErrorMemoryAllocation || grid_max == 1) return cuda_fail(ctx, e, "transfer scratch");
+        }
+    }
+    const size_t count_bytes = grid_max * row_counters;
     char *base = ctx->scratch.as<char>();
     int32_t *stage_col = reinterpret_cast<int32_t *>(base + at_col), *stage_cnt = reinterpret_cast<int32_t *>(base + at_cnt);
     uint32_t *counters = reinterpret_cast<uint32_t *>(base + at_counters);
@@ -1168,7 +1192,6 @@ int run_make_transfers(vrg_env *env, const float *dirs_local, int32_t k) {
         VRG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     }
     VRG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    if (ctx->scratch.bytes > kScratchKept) ctx->scratch.release();
     env->nnz = row_ptr[rows];
     env->have_transfers = true;
     return VRG_OK;

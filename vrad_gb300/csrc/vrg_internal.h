@@ -60,6 +60,18 @@ struct BounceGraph;   // bounce.cu: the scene's bounce loop as a graph
 
 constexpr size_t kScratchKept = (size_t)256 << 20;
 
+// Blocks that count transfer rows at once, `counters` bytes each: what the SMs
+// hold of 256 threads, but no more than 8 GiB of counters, and past kScratchKept
+// (which the context may keep anyway) only what lies outside the reserve.
+inline int64_t transfer_blocks(int64_t rows, int sms, uint64_t counters, uint64_t free_bytes, uint64_t reserve) {
+    uint64_t room = free_bytes > reserve ? free_bytes - reserve : 0;
+    room = room > kScratchKept ? room : kScratchKept;
+    room = room < (8ull << 30) ? room : 8ull << 30;
+    const uint64_t most = room / counters, want = (uint64_t)(rows < (int64_t)sms * 8 ? rows : (int64_t)sms * 8);
+    const uint64_t n = want < most ? want : most;
+    return n > 1 ? (int64_t)n : 1;
+}
+
 // k_few (trace.cu): queries of at most this many rays, a 64-bit key each, and
 // a counter per 32.
 constexpr int64_t kFewRays = 4096;
