@@ -327,11 +327,11 @@ struct Builder {
         deepest = std::max(deepest, stack + 4);
         uint32_t word[4];
         for (int c = 0; c < 4; c++) {
-            word[c] = kBvhLeafBit;
+            word[c] = bvh_leaf_word(0u, 1u);
             if (c >= n) continue;
             const Node2 &k = nodes[ch[c]];
             if (k.child[0] < 0)
-                word[c] = kBvhLeafBit | (uint32_t)k.first << 3 | (uint32_t)(k.count - 1);
+                word[c] = bvh_leaf_word((uint32_t)k.first, (uint32_t)k.count);
             else if (tasks && levels == 0)
                 tasks->push_back(Task{ch[c], stack + n - 1, at, c, {}});
             else
@@ -376,8 +376,8 @@ struct Builder {
 // `order` gets the finite triangles as the leaves list them, `nodes` the
 // four-wide tree over them, root first; an empty tree when there is none.  A
 // tree a walk's stack could not hold is built again by halving (depth of the
-// logarithm of the count).
-void build_bvh(const std::vector<float> &xyz, std::vector<int32_t> &order, std::vector<BvhNode> &nodes) {
+// logarithm of the count); false when that does not fit either.
+bool build_bvh(const std::vector<float> &xyz, std::vector<int32_t> &order, std::vector<BvhNode> &nodes) {
     Builder b;
     const int64_t n = (int64_t)xyz.size() / 9;
     b.threads = (int)std::min(16u, std::max(1u, std::thread::hardware_concurrency()));
@@ -407,7 +407,7 @@ void build_bvh(const std::vector<float> &xyz, std::vector<int32_t> &order, std::
     }
     order.clear();
     nodes.clear();
-    if (b.prims.empty()) return;
+    if (b.prims.empty()) return true;
     b.nodes.resize(2 * b.prims.size());
     if (many) b.spare.resize(b.prims.size());
     for (int pass = 0; pass < 2; pass++) {
@@ -450,9 +450,10 @@ void build_bvh(const std::vector<float> &xyz, std::vector<int32_t> &order, std::
         if (deepest <= kBvhStack) break;
         nodes.clear();
     }
-    if (nodes.empty()) return;
+    if (nodes.empty()) return false;
     order.resize(b.prims.size());
     for (size_t i = 0; i < order.size(); i++) order[i] = b.prims[i].id;
+    return true;
 }
 
 }  // namespace vrg

@@ -104,6 +104,7 @@ int vrg_env_setup_acceleration_structure(vrg_env *env) {
     vrg_ctx *ctx = env->ctx;
     const int64_t n = (int64_t)env->ids.size();
     if (n >= (int64_t)1 << 30) return fail(ctx, VRG_ERR_UNSUPPORTED, "more than 2^30 triangles");
+    if (!ctx->host_only && n > kBvhMax) return fail(ctx, VRG_ERR_UNSUPPORTED, "more than 2^29 triangles on a device");
     // the reference's tree is built when first asked for (vrg_env_tree_info /
     // vrg_env_get_tree): the device walks the walk tree
     scene_bounds(env->xyz, env->min_bound, env->max_bound);
@@ -145,9 +146,9 @@ int vrg_env_setup_acceleration_structure(vrg_env *env) {
     });
     // so is the hierarchy of the line queries (device contexts only)
     std::vector<BvhNode> bvh;
-    std::thread hierarchy([env, n, ctx, &bvh]() {
-        if (ctx->host_only || n >= (int64_t)1 << 27) return;
-        build_bvh(env->xyz, env->bvh_order, bvh);
+    bool bvh_fits = true;
+    std::thread hierarchy([env, ctx, &bvh, &bvh_fits]() {
+        if (!ctx->host_only) bvh_fits = build_bvh(env->xyz, env->bvh_order, bvh);
     });
     int rc = VRG_OK;
     if (on_device) {
@@ -275,6 +276,7 @@ int vrg_env_setup_acceleration_structure(vrg_env *env) {
         if (use_cells) nw += wall[f].size();
     // then the triangles in the order of the hierarchy's leaves
     hierarchy.join();
+    if (!bvh_fits) return fail(ctx, VRG_ERR_UNSUPPORTED, "hierarchy deeper than the walk's stack");
     const size_t nb = env->bvh_order.size(), tri_base = nr + nw;
     const size_t ne = tri_base + nb;
     // (the records of unused wall slots are zero, all others written below;

@@ -142,8 +142,8 @@ __device__ __forceinline__ bool bvh_pop(const uint2 *stk, int &sp, float best_t,
 template <int MODE, int OPT>
 __device__ __forceinline__ bool bvh_leaf(const DevScene &s, const BvhView &bv, const Ray &ray, float tmin, float tmax,
                                          int32_t skip, float any_limit, uint32_t word, int32_t &best, float &best_t) {
-    const size_t first = (size_t)bv.base + ((word & ~kBvhLeafBit) >> 3);
-    const uint32_t cnt = (word & 7u) + 1u;
+    const size_t first = (size_t)bv.base + bvh_leaf_first(word);
+    const uint32_t cnt = bvh_leaf_count(word);
     for (uint32_t i = 0; i < cnt; i++)
         if (tri_test<MODE, OPT>(s, ray, tmin, tmax, skip, any_limit, __ldg(s.leaf_planes + first + i), first + i, best, best_t))
             return true;

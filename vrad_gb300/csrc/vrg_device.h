@@ -84,10 +84,16 @@ __host__ __device__ inline const uint32_t *wall_table(const DevScene &s) {
 // children's bounds in steps of a power of two from an origin, one byte each
 // (bound[2 * axis] lower, [2 * axis + 1] upper, child c in byte c; a step or
 // more outside the child's box, which covers the rounding of bvh_step).  A
-// child word is a node index, or kBvhLeafBit | first record << 3 |
+// child word is a node index, or kBvhLeafBit | first record << 2 |
 // records - 1; an unused child is inside out.
 constexpr int kBvhLeaf = 4;
 constexpr uint32_t kBvhLeafBit = 1u << 31;
+constexpr int64_t kBvhMax = (int64_t)1 << 29;  // triangles that leaf words can number
+__host__ __device__ constexpr uint32_t bvh_leaf_word(uint32_t first, uint32_t count) {
+    return kBvhLeafBit | first << 2 | (count - 1u);
+}
+__host__ __device__ constexpr uint32_t bvh_leaf_first(uint32_t word) { return (word & ~kBvhLeafBit) >> 2; }
+__host__ __device__ constexpr uint32_t bvh_leaf_count(uint32_t word) { return (word & 3u) + 1u; }
 constexpr uint32_t kBvhNone = 0xffffffffu;
 constexpr int kBvhStack = 64;
 struct alignas(64) BvhNode {

@@ -290,7 +290,7 @@ void scene_bounds(const std::vector<float> &xyz, float *mn, float *mx);
 void build_kd_tree(const std::vector<float> &xyz, HostTree &tree, float *mn, float *mx);
 void build_walk_tree(const std::vector<float> &xyz, const float *mn, const float *mx,
                      const WalkTreeCosts &cost, HostTree &tree);
-void build_bvh(const std::vector<float> &xyz, std::vector<int32_t> &order, std::vector<BvhNode> &nodes);  // bvhbuild.cpp
+bool build_bvh(const std::vector<float> &xyz, std::vector<int32_t> &order, std::vector<BvhNode> &nodes);  // bvhbuild.cpp
 int build_walk_tree_device(vrg_env *env, HostTree &tree);  // kdbuild_gpu.cu
 void light_set_falloff(const vrg_light_keys &k, vrg_light &l);
 void light_parse_spot(const vrg_light_keys &k, vrg_light &l);
