@@ -19,7 +19,7 @@ def run(tmp_path, program, sources=()):
     main.write_text(program)
     cuda = build._cuda_home(build._nvcc())
     cmd = [cxx, "-O1", "-std=c++17", "-ffp-contract=off", "-I", str(CSRC), "-I", str(cuda / "include"), str(main),
-           *[str(CSRC / s) for s in sources], "-o", str(exe), "-L", str(cuda / "lib64"), "-lcudart", "-lpthread"]
+           *[str(CSRC / s) for s in sources], "-o", str(exe), "-L", str(cuda / "lib64"), "-lcudart", "-lpthread", "-ldl"]
     r = subprocess.run(cmd, capture_output=True, text=True)
     assert r.returncode == 0, r.stderr
     r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=300,

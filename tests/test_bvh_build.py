@@ -83,3 +83,56 @@ int main() {
 }
 """, ["bvhbuild.cpp"])
     assert out.split() == ["1"] * 15
+
+
+def test_threads_that_cannot_start_or_run_out_of_memory(tmp_path):
+    """No thread: the same tree on the caller's.  No memory, whichever allocation it is:
+    an exception that the caller gets."""
+    out = native.run(tmp_path, WALK + r"""
+#include <atomic>
+#include <cerrno>
+#include <new>
+#include <dlfcn.h>
+static std::atomic<bool> no_threads{false};
+static std::atomic<long> left{1l << 60};
+extern "C" int pthread_create(pthread_t *t, const pthread_attr_t *a, void *(*f)(void *), void *p) {
+    if (no_threads) return EAGAIN;
+    static auto real = (int (*)(pthread_t *, const pthread_attr_t *, void *(*)(void *), void *))dlsym(RTLD_NEXT, "pthread_create");
+    return real(t, a, f, p);
+}
+void *operator new(size_t n) {
+    if (left.fetch_sub(1) <= 0) throw std::bad_alloc();
+    if (void *p = malloc(n)) return p;
+    throw std::bad_alloc();
+}
+void operator delete(void *p) noexcept { free(p); }
+void operator delete(void *p, size_t) noexcept { free(p); }
+
+int main() {
+    const std::vector<float> xyz = soup(0, 40000);
+    std::vector<int32_t> order, other;
+    std::vector<BvhNode> nodes, same;
+    build_bvh(xyz, order, nodes);
+    no_threads = true;
+    build_bvh(xyz, other, same);
+    no_threads = false;
+    std::vector<char> seen(40000, 0);
+    bool all = other.size() == order.size() && deepest(same, seen) <= kBvhStack;
+    for (char c : seen) all = all && c == 1;
+    printf("%d\n", all);
+    int failed = 0;
+    for (long n = 0; n < 3000; n += n < 40 ? 1 : 97) {
+        std::vector<int32_t> o;
+        std::vector<BvhNode> k;
+        left = n;
+        try {
+            build_bvh(xyz, o, k);
+        } catch (const std::bad_alloc &) {
+            failed++;
+        }
+        left = 1l << 60;
+    }
+    printf("%d\n", failed > 30);
+}
+""", ["bvhbuild.cpp"])
+    assert out.split() == ["1", "1"]

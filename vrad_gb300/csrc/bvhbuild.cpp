@@ -16,6 +16,7 @@
 #include <limits>
 #include <thread>
 
+#include "vrg_crew.h"
 #include "vrg_internal.h"
 
 namespace vrg {
@@ -71,11 +72,11 @@ struct Bins {
 template <class F>
 void parallel(int parts, int32_t first, int32_t last, F f) {
     const int64_t n = last - first;
-    std::vector<std::thread> pool;
+    Crew crew;
     for (int p = 1; p < parts; p++)
-        pool.emplace_back([=, &f] { f(p, first + (int32_t)(n * p / parts), first + (int32_t)(n * (p + 1) / parts)); });
+        crew.run([=, &f] { f(p, first + (int32_t)(n * p / parts), first + (int32_t)(n * (p + 1) / parts)); });
     f(0, first, first + (int32_t)(n / parts));
-    for (std::thread &t : pool) t.join();
+    crew.join();
 }
 
 struct Builder {
@@ -270,7 +271,8 @@ struct Builder {
         const int32_t mid = leaf ? first : split(depth, first, last, nd.box, cb, leaf);
         if (!leaf) {
             if (depth < kForkDepth && nd.count > 1024 && threads > 1) {
-                std::thread left([&] { nd.child[0] = build(depth + 1, first, mid); });
+                Crew left;
+                left.run([&] { nd.child[0] = build(depth + 1, first, mid); });
                 nd.child[1] = build(depth + 1, mid, last);
                 left.join();
             } else {

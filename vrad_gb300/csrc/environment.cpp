@@ -9,6 +9,7 @@
 #include <thread>
 #include <vector>
 
+#include "vrg_crew.h"
 #include "vrg_internal.h"
 
 namespace vrg {
@@ -147,9 +148,9 @@ int vrg_env_setup_acceleration_structure(vrg_env *env) {
     // so is the hierarchy of the line queries (device contexts only)
     std::vector<BvhNode> bvh;
     bool bvh_fits = true;
-    std::thread hierarchy([env, ctx, &bvh, &bvh_fits]() {
-        if (!ctx->host_only) bvh_fits = build_bvh(env->xyz, env->bvh_order, bvh);
-    });
+    // joined where its order is needed, or on the way out
+    Crew hierarchy;
+    if (!ctx->host_only) hierarchy.run([env, &bvh, &bvh_fits] { bvh_fits = build_bvh(env->xyz, env->bvh_order, bvh); });
     int rc = VRG_OK;
     if (on_device) {
         const cudaError_t e = cudaSetDevice(ctx->device);
@@ -158,13 +159,6 @@ int vrg_env_setup_acceleration_structure(vrg_env *env) {
         build_walk_tree(env->xyz, env->min_bound, env->max_bound, env->walk_costs, env->walk_tree);
     }
     records.join();
-    // joined where its order is needed, or on the way out
-    struct Join {
-        std::thread &t;
-        ~Join() {
-            if (t.joinable()) t.join();
-        }
-    } join_hierarchy{hierarchy};
     if (rc != VRG_OK) return rc;
     // A walk pushes at most one subtree per inner node on its path, so a tree
     // whose paths hold fewer inner nodes than the device's stack has entries
@@ -275,7 +269,11 @@ int vrg_env_setup_acceleration_structure(vrg_env *env) {
     for (int f = 0; f < 6; f++)
         if (use_cells) nw += wall[f].size();
     // then the triangles in the order of the hierarchy's leaves
-    hierarchy.join();
+    try {
+        hierarchy.join();
+    } catch (const std::exception &e) {
+        return fail(ctx, VRG_ERR_NOMEM, std::string("hierarchy: ") + e.what());
+    }
     if (!bvh_fits) return fail(ctx, VRG_ERR_UNSUPPORTED, "hierarchy deeper than the walk's stack");
     const size_t nb = env->bvh_order.size(), tri_base = nr + nw;
     const size_t ne = tri_base + nb;
