@@ -380,6 +380,11 @@ int vrg_env_setup_acceleration_structure(vrg_env *env) {
     }
     env->built = true;
     env->cover_ready = false;
+    // what was made of an earlier tree names its leaf records
+    env->bvh_nodes = 0;
+    env->tile_tris = -1;
+    env->sky_n = 0;
+    env->sky_demand = 0;
     if (ctx->host_only) return VRG_OK;
     VRG_CUDA(ctx, cudaSetDevice(ctx->device));
     VRG_CUDA(ctx, env->d_few.reserve(kFewBytes));
