@@ -394,7 +394,7 @@ int vrg_batch_bake(vrg_batch *b, int32_t supersamples, uint64_t seed, int32_t ma
     float2 *rowabs = b->d_rowabs.as<float2>();
 
     // direct pass: one persistent launch over every scene, in the variant
-    // tuned for the batch's size (the register walk at 8 blocks per SM, or
+    // tuned for the batch's size in points (the register walk at 8 blocks per SM, or
     // the walk constants in shared memory at 9 or 8; the same results)
     using GatherKernel = void (*)(const BatchDesc *, const int64_t *, int, int, uint64_t, unsigned long long *,
                                   unsigned long long *);
@@ -421,7 +421,7 @@ int vrg_batch_bake(vrg_batch *b, int32_t supersamples, uint64_t seed, int32_t ma
         return e;
     };
     {
-        const int rc = tune_run(ctx, tune_key("batch_gather", tris, items), 3, gather);
+        const int rc = tune_run(ctx, tune_key("batch_gather", tris, all_points), 3, gather);
         if (rc != VRG_OK) return rc;
     }
 
