@@ -352,18 +352,15 @@ int vrg_batch_bake(vrg_batch *b, int32_t supersamples, uint64_t seed, int32_t ma
         const int rc = prepare_env(env);
         if (rc != VRG_OK) return rc;
     }
-    // the sky maps serve the launch when every scene has them
     std::vector<int64_t> points(E);
-    int64_t all_points = 0, repay = 0;
+    int64_t all_points = 0;
     for (int e = 0; e < E; e++) {
         const vrg_env *env = b->envs[e];
         points[e] = (env->luxel_offset.empty() ? 0 : env->luxel_offset.back()) * supersamples +
                     (int64_t)env->patches.leaf_patch.size();
         all_points += points[e];
-        repay += sky_map_points(env);
     }
-    bool map = true;
-    for (int e = 0; e < E; e++) map = use_sky_map(b->envs[e], points[e], all_points >= repay) && map;
+    const bool map = use_sky_maps(b->envs, points);
     std::vector<BatchDesc> descs(E);
     const auto whole_warps = [](int64_t n) { return (n + 31) & ~(int64_t)31; };
     std::vector<int64_t> seg(2 * E + 1, 0), rstart(E + 1, 0);

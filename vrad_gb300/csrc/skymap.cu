@@ -582,19 +582,56 @@ bool faces_in_sky_range(const vrg_env *env) {
 
 int64_t sky_map_points(const vrg_env *env) { return std::max<int64_t>(24 * env->geom.ntris, 40000); }
 
-bool use_sky_map(vrg_env *env, int64_t points, bool repaid) {
-    vrg_ctx *ctx = env->ctx;
-    bool ambient = false;
-    for (const vrg_light &l : env->lights) ambient = ambient || l.type == VRG_EMIT_SKYAMBIENT;
-    if (!ambient || env->sky_n < 0 || !env->faces_inside || !env->faces_in_sky_range) return false;
-    if (env->sky_n > 0) return true;
+bool wants_sky_map(const vrg_env *env) {
+    for (const vrg_light &l : env->lights)
+        if (l.type == VRG_EMIT_SKYAMBIENT) return true;
+    return false;
+}
+
+bool may_have_sky_map(const vrg_env *env) {
     const int64_t nt = env->geom.ntris;
+    return env->sky_n >= 0 && env->faces_inside && env->faces_in_sky_range && nt >= 1 && nt <= (int64_t)1 << 23 &&
+           env->geom.scale <= 16000.0f;
+}
+
+bool use_sky_map(vrg_env *env, int64_t points) {
+    if (!wants_sky_map(env) || !may_have_sky_map(env)) return false;
+    if (env->sky_n > 0) return true;
     // a build costs about what 24 sample points per triangle cost to walk, and
     // never less than 40,000 points: points walked so far count towards it, so
     // that a scene asked for a few at a time gets its maps when they repay
     env->sky_demand += points;
-    if (!repaid && env->sky_demand < sky_map_points(env)) return false;
-    if (nt < 1 || nt > (int64_t)1 << 23 || !(env->geom.scale <= 16000.0f)) return false;
+    return env->sky_demand >= sky_map_points(env) && have_sky_map(env);
+}
+
+bool use_sky_maps(const std::vector<vrg_env *> &envs, const std::vector<int64_t> &points) {
+    // the maps serve a launch over several scenes when all that want them have
+    // them, so none is built unless all can be, and all are paid for by the
+    // points that would else be walked, or by those walked so far
+    std::vector<vrg_env *> unbuilt;
+    int64_t asked = 0, repay = 0;
+    bool any = false, due = true;
+    for (size_t e = 0; e < envs.size(); e++) {
+        if (!wants_sky_map(envs[e])) continue;
+        if (!may_have_sky_map(envs[e])) return false;
+        any = true;
+        asked += points[e];
+        if (envs[e]->sky_n > 0) continue;
+        unbuilt.push_back(envs[e]);
+        envs[e]->sky_demand += points[e];
+        repay += sky_map_points(envs[e]);
+        due = due && envs[e]->sky_demand >= sky_map_points(envs[e]);
+    }
+    if (!any || !(due || asked >= repay)) return false;
+    for (vrg_env *env : unbuilt)
+        if (!have_sky_map(env)) return false;
+    return true;
+}
+
+bool have_sky_map(vrg_env *env) {
+    if (env->sky_n != 0) return env->sky_n > 0;
+    vrg_ctx *ctx = env->ctx;
+    const int64_t nt = env->geom.ntris;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(ctx->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return false;
     // three cells per direction and triangle: on the 8,208-triangle room a gather

@@ -306,9 +306,13 @@ int launch_trace_closest(vrg_env *env, const float *orig, const float *dir, cons
 int launch_test_lines(vrg_env *env, const float *start, const float *stop, int64_t n,
                       int32_t skip_id, float *frac);
 // Sky maps: whether the sky-ambient lines of `points` sample points on the
-// scene's faces go through the maps (built here when the points repay it), and
-// the maps as the kernels read them.
-bool use_sky_map(vrg_env *env, int64_t points, bool repaid = false);
+// scene's faces go through the maps (built here when the points repay it), the
+// same for a launch over several scenes, and the maps as the kernels read them.
+bool use_sky_map(vrg_env *env, int64_t points);
+bool use_sky_maps(const std::vector<vrg_env *> &envs, const std::vector<int64_t> &points);
+bool wants_sky_map(const vrg_env *env);     // it has a sky-ambient light
+bool may_have_sky_map(const vrg_env *env);  // its size and faces allow maps
+bool have_sky_map(vrg_env *env);            // built now if need be; false: no room, or under capture
 // The lookup rounds a depth by adding 1.5 * 2^23 to it, which keeps the order
 // down to -2^23 levels, 129 times the map's 65,000; farther out it wraps.
 bool faces_in_sky_range(const vrg_env *env);
