@@ -128,11 +128,16 @@ int vrg_ctx_reset_stats(vrg_ctx *ctx);
 int64_t vrg_ctx_launch_count(const vrg_ctx *ctx);
 
 /* Per-scene-size autotuning (no reference counterpart).  Tuned launch
- * sites ("direct_luxels", "transfer_rows", "bounce_spmv", "batch_gather") offer variants that give identical results (the bounce
- * variants: the same sums); the first launch in a bucket
+ * sites ("direct_luxels", "transfer_rows", "bounce_spmv", "batch_gather")
+ * offer variants that give identical results (the bounce variants: the same
+ * sums); the first launch in a bucket
  * "<site>/t<log2 triangles>/n<log2 work items>" times each twice on the real
- * input and keeps the fastest.  On by default; off, or inside a stream
- * capture, an untuned bucket runs variant 0. */
+ * input and keeps the fastest.  "direct_luxels" and "batch_gather" are for sky
+ * lines answered from maps, "transfer_rows" for rows that can be traced in
+ * tiles; "direct_luxels_walk", "batch_gather_walk" and "transfer_rows_walk" are
+ * the same sites without (a choice loaded under the plain name counts for both).
+ * On by default; off, or inside a stream capture, an untuned bucket runs
+ * variant 0. */
 int vrg_ctx_set_autotune(vrg_ctx *ctx, int enable);
 /* The variant chosen for `key` (-1 if untuned) and, when `ms` is not NULL,
  * up to `cap` per-variant times of the tuning run. */

@@ -418,7 +418,9 @@ int vrg_batch_bake(vrg_batch *b, int32_t supersamples, uint64_t seed, int32_t ma
         return e;
     };
     {
-        const int rc = tune_run(ctx, tune_key("batch_gather", tris, all_points), 3, gather);
+        // the maps and the walk are tuned apart
+        const std::string key = tune_key("batch_gather", tris, all_points);
+        const int rc = tune_run(ctx, map ? key : tune_key("batch_gather_walk", tris, all_points), 3, gather, key);
         if (rc != VRG_OK) return rc;
     }
 

@@ -246,7 +246,9 @@ int launch_gather_luxels(vrg_env *env, int ss, uint64_t seed, float *out_rgb,
         timing_end(ctx, "direct_luxels", ev);
         return e;
     };
-    return tune_run(ctx, tune_key("direct_luxels", env->geom.ntris, nlux * ss + npts), 12, launch);
+    // the maps and the walk are tuned apart
+    const std::string key = tune_key("direct_luxels", env->geom.ntris, nlux * ss + npts);
+    return tune_run(ctx, map ? key : tune_key("direct_luxels_walk", env->geom.ntris, nlux * ss + npts), 12, launch, key);
 }
 
 int launch_gather_points(vrg_env *env, const float *pts, const float *nrm, int64_t n,

@@ -1139,8 +1139,10 @@ int run_make_transfers(vrg_env *env, const float *dirs_local, int32_t k) {
             timing_end(ctx, "transfer_rows", ev);
             return e;
         };
-        const int rc = tune_run(ctx, tune_key("transfer_rows", env->geom.ntris, rows * (int64_t)k),
-                                kWalkVariants + (tiles ? kTileVariants : 0), launch);
+        // scenes and directions that cannot be traced in tiles are tuned apart
+        const std::string key = tune_key("transfer_rows", env->geom.ntris, rows * (int64_t)k);
+        const int rc = tune_run(ctx, tiles ? key : tune_key("transfer_rows_walk", env->geom.ntris, rows * (int64_t)k),
+                                kWalkVariants + (tiles ? kTileVariants : 0), launch, key);
         if (rc != VRG_OK) return rc;
         VRG_CUDA(ctx, cudaMemcpyAsync(h_nnz.data(), d_nnz, 4 * (size_t)nr, cudaMemcpyDeviceToHost, ctx->stream));
         VRG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));

@@ -8,6 +8,11 @@
 // keeps the fastest; later launches in that bucket use it directly.  Inside
 // a stream capture, or with tuning switched off, an untuned bucket runs
 // variant 0.
+//
+// A site whose work some scenes have done by another kind of kernel (sky maps or
+// walk, tiles or walk) keeps a bucket for each: the best of one says nothing
+// about the other.  A choice loaded from a file under the site's plain name
+// counts for both, as in files that know one bucket only.
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -33,12 +38,13 @@ std::string tune_key(const char *kernel, int64_t scene_size, int64_t work) {
 }
 
 int tune_pick(vrg_ctx *ctx, const std::string &key, int nvar,
-              const std::function<cudaError_t(int)> &launch, int *variant) {
+              const std::function<cudaError_t(int)> &launch, int *variant, const std::string &loaded_as) {
     *variant = 0;
     bool tune = false;
     {
         std::lock_guard<std::mutex> lk(ctx->mu);
         auto it = ctx->tuned.find(key);
+        if (it == ctx->tuned.end() && ctx->tune_loaded.count(loaded_as)) it = ctx->tuned.find(loaded_as);
         if (it != ctx->tuned.end()) *variant = it->second < nvar ? it->second : 0;
         else tune = ctx->autotune;
     }
@@ -80,10 +86,10 @@ int tune_pick(vrg_ctx *ctx, const std::string &key, int nvar,
 }
 
 int tune_run(vrg_ctx *ctx, const std::string &key, int nvar,
-             const std::function<cudaError_t(int)> &launch) {
+             const std::function<cudaError_t(int)> &launch, const std::string &loaded_as) {
     bool ran = false;
     int v = 0;
-    const int rc = tune_pick(ctx, key, nvar, [&](int i) { ran = true; return launch(i); }, &v);
+    const int rc = tune_pick(ctx, key, nvar, [&](int i) { ran = true; return launch(i); }, &v, loaded_as);
     if (rc != VRG_OK || ran) return rc;  // a tuning run already produced the result
     VRG_CUDA(ctx, launch(v));
     return VRG_OK;
@@ -135,7 +141,10 @@ int vrg_ctx_autotune_load(vrg_ctx *ctx, const char *path) {
     std::string key;
     int v;
     while (f >> key >> v)
-        if (v >= 0 && v < kTuneMaxVariants) ctx->tuned[key] = v;
+        if (v >= 0 && v < kTuneMaxVariants) {
+            ctx->tuned[key] = v;
+            ctx->tune_loaded.insert(key);
+        }
     return VRG_OK;
 }
 

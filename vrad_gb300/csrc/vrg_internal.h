@@ -6,6 +6,7 @@
 #include <cstdint>
 #include <functional>
 #include <map>
+#include <set>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -117,6 +118,7 @@ struct vrg_ctx {
     std::mutex scratch_mu;
     vrg::DevBuf scratch;
     std::map<std::string, int> tuned;                   // bucket key -> variant
+    std::set<std::string> tune_loaded;                  // keys whose choice came from a file
     std::map<std::string, std::vector<double>> tune_ms;  // bucket key -> variant times
 };
 
@@ -268,13 +270,14 @@ int cuda_fail(vrg_ctx *ctx, cudaError_t e, const char *what);
 
 // per-scene-size autotuning (tune.cpp).  tune_pick returns the bucket's
 // variant, first timing every variant through `launch` when the bucket is
-// new; tune_run then launches the chosen one unless tuning just did.
+// new; tune_run then launches the chosen one unless tuning just did.  Where the
+// bucket has no choice, one loaded from a file under `loaded_as` stands for it.
 std::string tune_key(const char *kernel, int64_t scene_size, int64_t work);
 constexpr int kTuneMaxVariants = 32;  // variants of one launch site, at most
 int tune_pick(vrg_ctx *ctx, const std::string &key, int nvar,
-              const std::function<cudaError_t(int)> &launch, int *variant);
+              const std::function<cudaError_t(int)> &launch, int *variant, const std::string &loaded_as = "");
 int tune_run(vrg_ctx *ctx, const std::string &key, int nvar,
-             const std::function<cudaError_t(int)> &launch);
+             const std::function<cudaError_t(int)> &launch, const std::string &loaded_as = "");
 
 // timing around kernel launches
 void timing_begin(vrg_ctx *ctx, const char *name, cudaEvent_t *start);
