@@ -418,20 +418,22 @@ void make_dirs(const vrg_env *env, int n, std::vector<SkyDir> &out) {
 
 static_assert(sizeof(SkyTri) == kSkyTriBytes && sizeof(SkyDir) == kSkyDirBytes, "SkyMapSizes counts them");
 
-// Whether `bytes` more leave the context's reserve free.
-bool leaves_reserve(vrg_ctx *ctx, size_t bytes) {
+// Device memory outside the context's reserve.
+size_t room_left(vrg_ctx *ctx) {
     size_t free_b = 0, total_b = 0;
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
         (void)cudaGetLastError();
-        return false;
+        return 0;
     }
     std::lock_guard<std::mutex> lk(ctx->mu);
-    return free_b >= bytes && free_b - bytes >= ctx->hbm_reserve;
+    return free_b > ctx->hbm_reserve ? free_b - ctx->hbm_reserve : 0;
 }
 
 // Builds env's maps with the context's scratch, which one build at a time
-// holds until its kernels are done.
-int build(vrg_env *env, int n) {
+// holds until its kernels are done.  The lists may take `room` bytes, or what is
+// left when they are counted (asking takes 15 us, so that is asked only where
+// `room` is too small).
+int build(vrg_env *env, int n, size_t room) {
     vrg_ctx *ctx = env->ctx;
     std::lock_guard<std::mutex> scratch(ctx->scratch_mu);
     DevBuf &tmp = ctx->scratch;
@@ -535,7 +537,7 @@ int build(vrg_env *env, int n) {
     VRG_CUDA(ctx, cudaMemcpyAsync(&entries, cursor, 8, cudaMemcpyDeviceToHost, st));
     VRG_CUDA(ctx, cudaStreamSynchronize(st));
     if (!sky_pool_indexable(entries)) return fail(ctx, VRG_ERR_UNSUPPORTED, "sky maps of more than 2^32 entries");
-    if (!leaves_reserve(ctx, 8 * (size_t)entries)) return fail(ctx, VRG_ERR_NOMEM, "no room for the sky maps' lists");
+    if (8 * (size_t)entries > room && 8 * (size_t)entries > room_left(ctx)) return fail(ctx, VRG_ERR_NOMEM, "no room for the sky maps' lists");
     VRG_CUDA(ctx, env->d_sky_pool.reserve(8 * (size_t)entries));
     g.pool = env->d_sky_pool.as<uint2>();
     VRG_CUDA(ctx, cells_pass(k_sky_cells<kFill>, k_sky_large<kFill>, 0, nt));
@@ -646,13 +648,14 @@ bool have_sky_map(vrg_env *env) {
     // the maps and their scratch inside what the context may take; the lists,
     // whose size the build finds out, are asked for there
     const SkyMapSizes sizes(nt, n, env->geom.has_sky != 0);
-    if (!leaves_reserve(ctx, sizes.kept + sizes.scratch)) return false;
+    const size_t room = room_left(ctx);
+    if (room < sizes.kept + sizes.scratch) return false;
     std::string said;
     {
         std::lock_guard<std::mutex> lk(ctx->mu);
         said = ctx->last_error;
     }
-    if (build(env, n) != VRG_OK) {
+    if (build(env, n, room - sizes.kept - sizes.scratch) != VRG_OK) {
         fail(ctx, 0, said);  // the call goes on without: its caller's last error stays
         (void)cudaGetLastError();
         env->d_sky_cells.release();
