@@ -556,7 +556,8 @@ __device__ __forceinline__ void trace_tile(const DevScene &s, const TileScene &t
                     }
                 }
                 __syncwarp();
-                bfar[r] = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(best_t[r])));
+                // (as numbers that order the same: a hit at -0 counts as +0)
+                bfar[r] = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(radd(best_t[r], 0.0f))));
             }
             far = bfar[0];
 #pragma unroll
