@@ -48,9 +48,10 @@ def _alone(made):
 def test_a_scene_without_sky_light_among_others(gpu_ctx):
     made = [_scene(gpu_ctx, 80 + i, sky=i != 1) for i in range(3)]
     alone = _alone([_scene(gpu_ctx, 80 + i, sky=i != 1) for i in range(3)])
-    first, got = _bake(gpu_ctx, made)
-    again, same = _bake(gpu_ctx, made)
-    assert first > 0 and again == 0
+    passes = [_bake(gpu_ctx, made) for _ in range(6)]  # enough points to repay the maps
+    built = [maps > 0 for maps, _ in passes]
+    assert sum(built) == 1 and not built[-1]
+    got, same = passes[0][1], passes[-1][1]
     for want, a, b in zip(alone, got, same):
         assert np.abs(want).max() > 0
         assert bits_equal(a["luxels"], want) and bits_equal(b["luxels"], want)
@@ -58,7 +59,8 @@ def test_a_scene_without_sky_light_among_others(gpu_ctx):
 
 def test_none_is_built_where_one_cannot_be(gpu_ctx):
     made = [_scene(gpu_ctx, 90 + i, outside=i == 2) for i in range(3)]
-    maps, got = _bake(gpu_ctx, made)
-    assert maps == 0
+    for _ in range(6):
+        maps, got = _bake(gpu_ctx, made)
+        assert maps == 0
     for want, a in zip(_alone(made), got):
         assert bits_equal(a["luxels"], want)
