@@ -108,7 +108,7 @@ __device__ int32_t filtered_trace(const DevScene &s, const Ray &ray, const RayPr
                     filtered_tri(s, ray, tmin, tmax, skip, __ldg(s.leaf_planes + start + j), (size_t)start + j, f,
                                  st.best, st.best_t);
             }
-            if (!pop_next<kClosest>(st.stk, sp, st.best_t, st.node, st.t0, st.t1)) break;
+            if (!pop_next(st.stk, sp, st.best_t, st.node, st.t0, st.t1)) break;
             st.sp = sp;
         }
     }

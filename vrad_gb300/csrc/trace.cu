@@ -122,12 +122,12 @@ __global__ void __launch_bounds__(kThreads, MINB) k_bvh(DevScene s, BvhView bv, 
         if (inner == 0u || __popc(leaves) >= LEAVES) {
             if (at_leaf)
                 done = bvh_leaf<MODE, OPT>(s, bv, ray, t0, len, q.skip, any_limit, cur, best, best_t) ||
-                       !bvh_pop<MODE>(stk, sp, best_t, cur);
+                       !bvh_pop(stk, sp, best_t, cur);
         } else {
 #pragma unroll
             for (int u = 0; u < STEPS; u++)
                 if (active && !done && !(cur & kBvhLeafBit))
-                    if (!bvh_step<ORDER>(bv, rp, t0, fminf(len, best_t), stk, sp, cur)) done = !bvh_pop<MODE>(stk, sp, best_t, cur);
+                    if (!bvh_step<ORDER>(bv, rp, t0, fminf(len, best_t), stk, sp, cur)) done = !bvh_pop(stk, sp, best_t, cur);
         }
         if (done) {
             active = false;

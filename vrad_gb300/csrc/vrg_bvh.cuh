@@ -126,12 +126,11 @@ __device__ __forceinline__ bool bvh_step(const BvhView &bv, const BoxRay &rp, fl
 
 // The next stacked node that can still hold the answer; false when there is
 // none.
-template <int MODE>
 __device__ __forceinline__ bool bvh_pop(const uint2 *stk, int &sp, float best_t, uint32_t &cur) {
     while (sp > 0) {
         sp--;
         const uint2 e = stk[sp];
-        if (MODE != kAny && __uint_as_float(e.y) > best_t) continue;
+        if (__uint_as_float(e.y) > best_t) continue;
         cur = e.x;
         return true;
     }
@@ -169,7 +168,7 @@ __device__ __forceinline__ int32_t bvh_trace(const DevScene &s, const BvhView &b
             } else {
                 more = bvh_step<MODE == kClosest>(bv, rp, tmin, fminf(tmax, best_t), stk, sp, cur);
             }
-            if (!more && !bvh_pop<MODE>(stk, sp, best_t, cur)) break;
+            if (!more && !bvh_pop(stk, sp, best_t, cur)) break;
         }
     }
     *t_out = best_t;

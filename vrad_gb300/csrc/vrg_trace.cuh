@@ -142,12 +142,11 @@ __device__ __forceinline__ void clip_box(const float *mn, const float *mx, float
 }
 
 // Modes of a walk:
-//   kAny      stop at the first accepted triangle;
 //   kClosest  minimum t, ties to the lower triangle index -- the same answer
 //             as testing every triangle;
 //   kSkyOcc   closest-hit, except that a hit with t < any_limit stops at
 //             once (the caller guarantees no sky triangle can be hit there).
-enum TraceMode { kAny = 0, kClosest = 1, kSkyOcc = 2 };
+enum TraceMode { kClosest = 1, kSkyOcc = 2 };
 
 // Resumable state of one walk: the current subtree and its t interval, the
 // stack of far subtrees, and the best hit so far.
@@ -230,8 +229,7 @@ __device__ __forceinline__ bool inner_step(const RayPre &rp, uint2 nd, float &t0
 //   hit iff all three are >= 0.
 // Tests TriangleIndexList entry k, whose plane w0 the caller has loaded, and
 // updates best / best_t (minimum t, ties to the lower index).  Returns true
-// when the walk ends here: any accepted hit in kAny mode, a hit before
-// any_limit in kSkyOcc mode.  The edge part is fetched only when the plane
+// when the walk ends here: a hit before any_limit in kSkyOcc mode.  The edge part is fetched only when the plane
 // hit is in range.
 // Leaf-record load; kOptStream asks L1 not to keep the line (the leaf records
 // of a large scene stream past L1, where they would evict the nodes and the
@@ -263,7 +261,7 @@ __device__ __forceinline__ bool tri_test(const DevScene &s, const Ray &ray, floa
     }
     const float t = rdiv(num, den);
     if (!(t >= tmin && t < tmax)) return false;
-    if (MODE != kAny && !(t <= best_t)) return false;
+    if (!(t <= best_t)) return false;
     const float4 *ed = s.leaf_edges + 2 * k;
     const float4 w2 = leaf_load<OPT>(ed + 1);
     if (__float_as_int(w2.z) == skip) return false;
@@ -283,7 +281,7 @@ __device__ __forceinline__ bool tri_test(const DevScene &s, const Ray &ray, floa
     const float b2 = rsub(rsub(1.0f, b0), b1);
     if (b0 >= 0.0f && b1 >= 0.0f && b2 >= 0.0f) {
         const int32_t ti = (int32_t)(idx_drop >> 2);
-        if (MODE == kAny || (MODE == kSkyOcc && t < any_limit)) {
+        if (MODE == kSkyOcc && t < any_limit) {
             best = ti;
             best_t = t;
             return true;
@@ -320,15 +318,14 @@ __device__ __forceinline__ bool leaf_test(const DevScene &s, const Ray &ray, flo
     return false;
 }
 
-// Pops the next stacked subtree whose interval can still hold the answer
-// (kAny: every one); false when the stack is empty.
-template <int MODE>
+// Pops the next stacked subtree whose interval can still hold the answer;
+// false when the stack is empty.
 __device__ __forceinline__ bool pop_next(const uint4 *stk, int &sp, float best_t,
                                          uint32_t &node, float &t0, float &t1) {
     while (sp > 0) {
         --sp;
         const uint4 e = stk[sp];
-        if (MODE != kAny && __uint_as_float(e.y) > best_t) continue;
+        if (__uint_as_float(e.y) > best_t) continue;
         node = e.x;
         t0 = __uint_as_float(e.y);
         t1 = __uint_as_float(e.z);
@@ -359,7 +356,7 @@ __device__ __forceinline__ bool trace_step(const DevScene &s, const Ray &ray, co
     if (reached && leaf_test<MODE, LB, OPT>(s, ray, tmin, tmax, skip, any_limit, nd.x >> 2,
                                             (int)__uint_as_float(nd.y), st.best, st.best_t))
         return true;
-    if (!pop_next<MODE>(st.stk, sp, st.best_t, st.node, st.t0, st.t1))
+    if (!pop_next(st.stk, sp, st.best_t, st.node, st.t0, st.t1))
         return true;
     st.sp = sp;
     return false;
