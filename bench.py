@@ -297,18 +297,14 @@ def _trace_roofline(kernel, units, avg_ms, bytes_per_unit, hbm_peak, hbm_kind, l
     """Roofline record of a traversal kernel: the governing roof is
     instruction issue.  Beside it the bytes that a kd walk of the same lines
     would read (nodes and leaf records) against the L2 rate, and HBM from the
-    DRAM bytes ncu counted for the same kernel.  The instruction
-    count is the tuned variant's own (`warp_instructions_per_unit_v<n>`)
-    where the summary has it."""
+    DRAM bytes ncu counted for the same kernel, the instruction count
+    and the bytes being the tuned variant's own (`..._v<n>` in the summary)."""
     alg = bytes_per_unit * units / (avg_ms * 1e-3) / 1e9
-    traffic = _profile_value(prof, f"dram_bytes_per_launch_full_v{variant}") if variant is not None else None
-    if traffic is None:
-        traffic = _ncu_traffic(prof)
+    per = "" if variant is None else f"_v{variant}"  # another variant's counts say nothing
+    traffic = _ncu_traffic(prof) if variant is None else _profile_value(prof, f"dram_bytes_per_launch_full{per}")
     sm_mhz = (clk or {}).get("sm_mhz")
-    inst = _profile_value(prof, f"warp_instructions_per_unit_v{variant}") if variant is not None else None
-    inst_of = f"variant {variant}" if inst is not None else "the variant the summary names"
-    if inst is None:
-        inst = _profile_value(prof, "warp_instructions_per_unit")
+    inst = _profile_value(prof, f"warp_instructions_per_unit{per}")
+    inst_of = f"variant {variant}" if variant is not None else "the kernel"
     issue = issue_roofline(inst, units, avg_ms, sm_mhz, sms, f"profiles/{prof}")
     if issue:
         issue["instructions_of"] = inst_of
@@ -328,9 +324,8 @@ def _trace_roofline(kernel, units, avg_ms, bytes_per_unit, hbm_peak, hbm_kind, l
     if issue:
         rec.update({"achieved": issue["achieved"], "peak": issue["peak"], "unit": issue["unit"],
                     "frac": issue["frac"], "issue": issue})
-    else:
-        rec.update({"achieved": rec["walk_l2"]["achieved"], "peak": rec["walk_l2"]["peak"], "unit": "GB/s",
-                    "frac": rec["walk_l2"]["frac"], "bound": "l2"})
+    else:  # no count of this variant: no fraction of a roof
+        rec.update({"achieved": None, "peak": None, "unit": "", "frac": None})
     return rec
 
 
