@@ -263,7 +263,9 @@ int vrg_env_get_triangle_vertices(const vrg_env *env, int64_t first, int64_t n, 
  * they stay resident.  The reference's own tree (its candidates, costs and
  * partition order) is built when vrg_env_tree_info or vrg_env_get_tree first
  * asks for it.  Both trees give the same answers: every query returns what
- * testing every triangle would. */
+ * testing every triangle would.  VRG_ERR_UNSUPPORTED past 2^29 triangles on a
+ * device (2^30 on the host), VRG_ERR_NOMEM when the line queries' hierarchy
+ * cannot be built. */
 int vrg_env_setup_acceleration_structure(vrg_env *env);
 int64_t vrg_env_num_triangles(const vrg_env *env);
 /* Size of the reference's tree: nodes, triangle-index-list length, height. */
@@ -559,7 +561,8 @@ typedef struct vrg_server vrg_server;
  * not fit with the context's HBM reserve to spare). */
 int vrg_env_relight_prepare(vrg_env *env, int32_t supersamples, uint64_t seed,
                             int32_t max_bounces, float rel_tol);
-/* Device memory that admission keeps free for other work (default 1 GiB). */
+/* Device memory that admission, the sky maps, and the transfer build's counters
+ * past 256 MiB keep free for other work (default 1 GiB). */
 int vrg_ctx_set_hbm_reserve(vrg_ctx *ctx, uint64_t bytes);
 /* Apply light edits and update the scene: luxels and leaf points of the faces
  * within the old or new radius of an edited light are re-gathered (the same

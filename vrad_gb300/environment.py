@@ -90,7 +90,8 @@ class Context:
               "set_transfer_table_limit")
 
     def set_hbm_reserve(self, nbytes: int):
-        """Device memory that relight admission keeps free (default 1 GiB)."""
+        """Device memory that relight admission, the sky maps and the transfer build's
+        larger counters keep free (default 1 GiB)."""
         check(self.lib.vrg_ctx_set_hbm_reserve(self.h, int(nbytes)), self.h, "set_hbm_reserve")
 
     def set_autotune(self, on: bool):
