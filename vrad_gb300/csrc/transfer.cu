@@ -1040,11 +1040,13 @@ int run_make_transfers(vrg_env *env, const float *dirs_local, int32_t k) {
     const int vthreads[kWalkVariants + kTileVariants] = {256, 256, 512, 512, 256, 128};
     const int tbundles[kTileVariants] = {4, 2, 2};
     const size_t tile_smem = smem + 28 * (size_t)ts.nclusters;
+    // (a kernel's limit is the process's, not the call's: always the largest that
+    // a scene can need, so that no thread lowers another's)
+    constexpr int kSmemMax = 4 * kBitmapShared, kTileSmemMax = kSmemMax + 28 * kClusterMax;
     for (const RowKernel kern : kvar)
-        VRG_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    if (tiles)
-        for (const TileKernel kern : tvar)
-            VRG_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_smem));
+        VRG_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax));
+    for (const TileKernel kern : tvar)
+        VRG_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kTileSmemMax));
     // rows go through in chunks whose staging stays near 1 GiB
     const int64_t chunk =
         std::max<int64_t>(1, std::min<int64_t>(rows, ((int64_t)1 << 30) / (8 * (int64_t)tsize)));
