@@ -7,7 +7,9 @@
 // the box centres (every split of the widest axis for the last few triangles),
 // down to leaves of at most kBvhLeaf triangles; the binary
 // tree is then collapsed by opening the child of largest surface until a node
-// has four.  On the 12,300-triangle room an any-hit line visits 17 four-wide
+// has four.  Child boxes are kept as bytes on a grid of the node (as in Ylitie, Karras
+// and Laine, "Efficient incoherent ray traversal on GPUs through compressed
+// wide BVHs", 2017).  On the 12,300-triangle room an any-hit line visits 17 four-wide
 // nodes and 0.3 triangles where the kd walk visits 51 nodes and 6.3.
 #include <algorithm>
 #include <atomic>
